@@ -17,7 +17,7 @@
 #include "ilc_device.cuh"
 #include "ilc_internal.h"
 #include "ilc_quantity.cuh"
-#include "ilc_walk4.cuh"
+#include "ilc_raylist.cuh"
 
 namespace ilc {
 
@@ -154,77 +154,39 @@ __global__ void loss_seed_kernel(const float* __restrict__ img, const float* __r
   if ((threadIdx.x & 31) == 0) atomicAdd(loss, part);
 }
 
-// d e / d v_p = w_p / sum(w) for the 8 slots of one evaluation (0 where the
-// finalize has no weight): scatter4 adds c * that to grad at the sorted
-// particle index of point J's slots. The accumulator is double: a cell's
-// gradient sums contributions of both signs from many rays, and fp32
-// accumulation loses digits to cancellation.
-template <int J>
-__device__ __forceinline__ void scatter4(const Step4& s, float c, double* __restrict__ grad) {
-  if (c == 0.0f) return;
-  float w[8];
-  float ws = 0.0f;
-#pragma unroll
-  for (int t = 0; t < 8; ++t) {
-    w[t] = weight3d(s4_d(s, J, t));
-    ws = ws + w[t];
-  }
-  if (!(ws > 0.0f) || !isfinite(ws)) return;
-  const double f = (double)c / (double)ws;
-#pragma unroll
-  for (int t = 0; t < 8; ++t) {
-    const int id = __float_as_int(s4_v(s, J, t));
-    if (id >= 0 && w[t] != 0.0f) atomicAdd(&grad[id], f * (double)w[t]);
-  }
-}
-
-// Point 2's slots of the previous step (it is the next step's k1).
-struct PrevSlots {
-  float d[8];
+// A point's slots as the scatter needs them: d e / d v_p = w_p / sum(w).
+struct ScatterSlots {
+  float w[8], ws;
   int id[8];
 };
 
-__device__ __forceinline__ void scatter_prev(const PrevSlots& s, float c,
-                                             double* __restrict__ grad) {
-  if (c == 0.0f) return;
-  float w[8];
-  float ws = 0.0f;
+__device__ __forceinline__ void scatter_slots(const PointSlots& s, ScatterSlots& o) {
+  slot_weights(s, o.w, o.ws);
 #pragma unroll
-  for (int t = 0; t < 8; ++t) {
-    w[t] = weight3d(s.d[t]);
-    ws = ws + w[t];
-  }
-  if (!(ws > 0.0f) || !isfinite(ws)) return;
-  const double f = (double)c / (double)ws;
+  for (int t = 0; t < 8; ++t) o.id[t] = __float_as_int(s.v[t]);
+}
+
+// Adds c * w_p / sum(w) to grad at the slots' sorted particle indices (nothing
+// where the finalize has no weight). The accumulator is double: a cell's
+// gradient sums contributions of both signs from many rays, and fp32
+// accumulation loses digits to cancellation.
+__device__ __forceinline__ void scatter(const ScatterSlots& s, double c,
+                                        double* __restrict__ grad) {
+  if (c == 0.0 || !(s.ws > 0.0f) || !isfinite(s.ws)) return;
+  const double f = c / (double)s.ws;
 #pragma unroll
   for (int t = 0; t < 8; ++t)
-    if (s.id[t] >= 0 && w[t] != 0.0f) atomicAdd(&grad[s.id[t]], f * (double)w[t]);
+    if (s.id[t] >= 0 && s.w[t] != 0.0f) atomicAdd(&grad[s.id[t]], f * (double)s.w[t]);
 }
 
-__device__ __forceinline__ void keep_prev(const Step4& s, PrevSlots& p) {
-#pragma unroll
-  for (int t = 0; t < 8; ++t) {
-    p.d[t] = s4_d(s, 2, t);
-    p.id[t] = __float_as_int(s4_v(s, 2, t));
-  }
-}
-
-// nn8 value of point J (finalize order) with the values read by index.
-template <int J>
-__device__ __forceinline__ float value_by_id(const Step4& s, const float4* __restrict__ parts) {
-  float w[8];
-#pragma unroll
-  for (int t = 0; t < 8; ++t) w[t] = weight3d(s4_d(s, J, t));
-  float ws = 0.0f;
-#pragma unroll
-  for (int t = 0; t < 8; ++t) ws = ws + w[t];
+// nn8 value of a point (finalize order) with the values read by index.
+__device__ __forceinline__ float value_by_id(const ScatterSlots& s,
+                                             const float4* __restrict__ parts) {
   float dot = 0.0f;
 #pragma unroll
-  for (int t = 0; t < 8; ++t) {
-    const int id = __float_as_int(s4_v(s, J, t));
-    dot = __fmaf_rn(w[t], id >= 0 ? __ldg(&parts[id].w) : 0.0f, dot);
-  }
-  return (ws != 0.0f && dot != 0.0f) ? dot / ws : 0.0f;
+  for (int t = 0; t < 8; ++t)
+    dot = __fmaf_rn(s.w[t], s.id[t] >= 0 ? __ldg(&parts[s.id[t]].w) : 0.0f, dot);
+  return (s.ws != 0.0f && dot != 0.0f) ? dot / s.ws : 0.0f;
 }
 
 struct AdjK {
@@ -240,107 +202,136 @@ struct AdjK {
   const float* __restrict__ seed;  // dL/dI_raw per pixel (whole image)
   double* __restrict__ grad;       // dL/dq per sorted particle
   int row0, row_end;               // pixel rows of this launch; rec_* indexed from row0
-  unsigned* queue;                 // persistent launch: tile counter (nullptr: block per tile)
-  unsigned ntiles, tiles_x;
+  unsigned long long* queue;       // ray counter
+  unsigned long long n_rays;       // 128 per 16 x 8 tile
+  unsigned tiles_x;
+  float4* over;                    // list overflow, kOver per resident ray
 };
 
-// The rays of one 16 x 8 tile (one per thread; no block synchronisation).
-__device__ __forceinline__ void adjoint_tile(const AdjK& a, const GridView& g,
-                                             const char4* __restrict__ spiral, SlotMem& slot_mem,
-                                             uint32_t* __restrict__ flags,
-                                             unsigned long long* __restrict__ stats, int bx,
-                                             int by) {
-  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
-  const int ix = bx * 16 + (warp & 1) * 8 + (lane & 7);
-  const int iy = a.row0 + by * 8 + (warp >> 1) * 4 + (lane >> 3);
-  if (ix >= a.cam.nx || iy >= a.row_end) return;
-  const int64_t ray = (int64_t)(iy - a.row0) * a.cam.nx + ix;  // in the launch's rows
-  const float gi = a.seed[(int64_t)iy * a.cam.nx + ix];
-  if (gi == 0.0f) return;
-  float px, py, pz;
-  pixel_corner(a.cam, ix, iy, px, py, pz);
+constexpr int kAdjBlocks = 4;
+
+struct AdjMem {
+  char4 spiral[1000];
+  WarpLists lists[kListWarps];
+};
+
+// Four lanes per ray, as in the render kernel: lane j scatters point j (point
+// 3 only enters the error estimate, and a checkpointed replay does not need
+// it). Point 2 of an accepted step is the next one's k1: its lane holds its
+// slots back until the next step's size is known and scatters both terms at
+// once.
+__global__ void __launch_bounds__(kListThreads, kAdjBlocks)
+adjoint_kernel(const __grid_constant__ AdjK a, const __grid_constant__ GridView g,
+               const char4* __restrict__ spiral_g, uint32_t* __restrict__ flags,
+               unsigned long long* __restrict__ stats) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  AdjMem& M = *reinterpret_cast<AdjMem*>(smem_raw);
+  load_spiral(M.spiral, spiral_g);
+  const int lane = threadIdx.x & 31;
+  const int r = lane >> 2, pj = lane & 3;
+  WarpLists& W = M.lists[threadIdx.x >> 5];
+  const unsigned wg = blockIdx.x * kListWarps + (threadIdx.x >> 5);
+  if (lane == 0) W.over = a.over + (size_t)wg * kRays * kOver;
+  const float ext0 = 0.06f * g.cs0;
   const float lx = a.cam.look0, ly = a.cam.look1, lz = a.cam.look2;
-  WalkStats ws;
+  const float fa = (float)a.atol, fr = (float)a.rtol;
+  const bool replay = a.mode == ILC_ADJOINT_CHECKPOINT;
+  bool have = false, drained = false, fresh = true;
+  float px = 0.0f, py = 0.0f, pz = 0.0f, gi = 0.0f;
+  float I = 0.0f, z = 0.0f, h = 1.0f, k1 = 0.0f;
+  int64_t limit = 0;
+  const float* hs = nullptr;
   unsigned long long steps = 0;
-  PrevSlots prev;
   bool have_prev = false;
-  float z = a.z0;
-  if (a.mode == ILC_ADJOINT_CHECKPOINT) {
-    const int32_t n = a.rec_n[ray];
-    const float* hs = a.rec_h + ray * a.rec_cap;
-    for (int32_t i = 0; i < n; ++i) {
-      const float h = hs[i];
-      float p[4];
-      rkf_points(z, h, p);
-      Step4 s;
-      s4_bind(s, slot_mem);
-      nn8_walk_step4<true>(g, spiral, px, py, pz, lx, ly, lz, p, s, ws);
-      scatter4<0>(s, gi * (h * 1408.f / 2565.f), a.grad);
-      scatter4<1>(s, gi * (h * 2197.f / 4101.f), a.grad);
-      scatter4<2>(s, gi * (-h / 5.f), a.grad);
-      if (have_prev) scatter_prev(prev, gi * (h * 25.f / 216.f), a.grad);
-      keep_prev(s, prev);
-      have_prev = true;
-      z += h;
-      ++steps;
+  ScatterSlots prev;
+  double prev_c = 0.0;
+  WalkStats ws;
+  for (;;) {
+    for (;;) {
+      const unsigned want = __ballot_sync(kAll, !have && !drained && pj == 0);
+      if (!want) break;
+      const unsigned long long q = take_rays(a.queue, want, fresh, lane, wg);
+      fresh = false;
+      if (!have && !drained) {
+        drained = q >= a.n_rays;
+        if (!drained) {
+          const unsigned tile = (unsigned)(q >> 7), t = (unsigned)(q & 127u);
+          const int sub = (int)(t >> 3);
+          const int ix = (int)(tile % a.tiles_x) * 16 + (sub & 3) * 4 + (int)(t & 3u);
+          const int iy =
+              a.row0 + (int)(tile / a.tiles_x) * 8 + (sub >> 2) * 2 + (int)((t >> 2) & 1u);
+          if (ix < a.cam.nx && iy < a.row_end) {
+            gi = a.seed[(int64_t)iy * a.cam.nx + ix];
+            have = gi != 0.0f;
+            const int64_t ray = (int64_t)(iy - a.row0) * a.cam.nx + ix;  // in the launch's rows
+            pixel_corner(a.cam, ix, iy, px, py, pz);
+            limit = replay ? a.rec_n[ray] : a.max_steps;
+            hs = replay ? a.rec_h + ray * a.rec_cap : nullptr;
+          }
+        }
+        if (have) {
+          I = 0.0f;
+          k1 = 0.0f;
+          z = a.z0;
+          h = 1.0f;
+          steps = 0;
+          have_prev = false;
+          if (pj == 0) ray_reset(W.meta[r], ext0);
+        }
+      }
+      __syncwarp();
     }
-  } else {
-    // Recompute: run the forward controller again; accepted steps scatter.
-    float I = 0.0f, h = 1.0f, k1 = 0.0f;
-    float pts[4];
-    rkf_points(z, h, pts);
-    const float fa = (float)a.atol, fr = (float)a.rtol;
-    while (z < a.z_end) {
-      if ((int64_t)steps >= a.max_steps) { atomicOr(flags, FLAG_STEP_LIMIT); break; }
-      Step4 s;
-      s4_bind(s, slot_mem);
-      nn8_walk_step4<true>(g, spiral, px, py, pz, lx, ly, lz, pts, s, ws);
-      const float e[4] = {value_by_id<0>(s, g.parts), value_by_id<1>(s, g.parts),
-                          value_by_id<2>(s, g.parts), value_by_id<3>(s, g.parts)};
-      const float zb = z, hb = h;
-      if (a.controller == ILC_CONTROLLER_REF32)
-        rkf_advance_ref32(I, z, h, k1, fa, fr, a.z_end, e, kEps, kHmin, kHmax, pts);
-      else
-        rkf_advance_fp64(I, z, h, k1, a.atol, a.rtol, a.z_end, e, kEps, kHmin, kHmax, pts);
-      ++steps;
-      if (z != zb) {
-        scatter4<0>(s, gi * (hb * 1408.f / 2565.f), a.grad);
-        scatter4<1>(s, gi * (hb * 2197.f / 4101.f), a.grad);
-        scatter4<2>(s, gi * (-hb / 5.f), a.grad);
-        if (have_prev) scatter_prev(prev, gi * (hb * 25.f / 216.f), a.grad);
-        keep_prev(s, prev);
+    if (!__any_sync(kAll, have)) break;
+    const bool go = have && (int64_t)steps < limit && (replay || z < a.z_end);
+    if (go && replay) h = hs[steps];
+    const float zq = step_point(z, h, pj);
+    PointSlots s;
+    eval_points<true>(g, M.spiral, W, lane, go && !(replay && pj == 3), px, py, pz, lx,
+                               ly, lz, zq, s, ws);
+    ScatterSlots cur;
+    if (go) scatter_slots(s, cur);
+    bool accepted = go;
+    const float hb = h;
+    if (replay) {
+      if (go) z += h;
+    } else {
+      float e[4];
+      share4(go ? value_by_id(cur, g.parts) : 0.0f, lane, e);
+      if (go) {
+        const float zb = z;
+        float next[4];
+        if (a.controller == ILC_CONTROLLER_REF32)
+          rkf_advance_ref32(I, z, h, k1, fa, fr, a.z_end, e, kEps, kHmin, kHmax, next);
+        else
+          rkf_advance_fp64(I, z, h, k1, a.atol, a.rtol, a.z_end, e, kEps, kHmin, kHmax, next);
+        accepted = z != zb;
+      }
+    }
+    if (go) ++steps;
+    if (accepted) {
+      if (pj < 2) {
+        scatter(cur, (double)(gi * (pj == 0 ? hb * 1408.f / 2565.f : hb * 2197.f / 4101.f)),
+                a.grad);
+      } else if (pj == 2) {
+        if (have_prev) scatter(prev, prev_c + (double)(gi * (hb * 25.f / 216.f)), a.grad);
+        prev = cur;
+        prev_c = (double)(gi * (-hb / 5.f));
         have_prev = true;
       }
     }
+    const bool fin = have && (!go || (replay ? (int64_t)steps >= limit : !(z < a.z_end)));
+    if (fin) {
+      if (pj == 2 && have_prev) scatter(prev, prev_c, a.grad);
+      if (pj == 0) {
+        if (!replay && z < a.z_end) atomicOr(flags, FLAG_STEP_LIMIT);
+        atomicAdd(&stats[0], steps);
+      }
+      have = false;
+    }
+    __syncwarp();
   }
-  unsigned long long c = ws.cells, k = ws.cands;
-  atomicAdd(&stats[0], steps);
-  atomicAdd(&stats[3], c);
-  atomicAdd(&stats[4], k);
-}
-
-// Persistent: the resident blocks take tiles from a queue (one block per tile
-// without one), as the render kernel does.
-__global__ void __launch_bounds__(128)
-adjoint_kernel(AdjK a, GridView g, const char4* __restrict__ spiral_g,
-               uint32_t* __restrict__ flags, unsigned long long* __restrict__ stats) {
-  __shared__ char4 spiral[1000];
-  __shared__ SlotMem slot_mem;
-  __shared__ unsigned next_tile;
-  load_spiral(spiral, spiral_g);
-  if (!a.queue) {
-    adjoint_tile(a, g, spiral, slot_mem, flags, stats, blockIdx.x, blockIdx.y);
-    return;
-  }
-  for (;;) {
-    if (threadIdx.x == 0) next_tile = atomicAdd(a.queue, 1u);
-    __syncthreads();
-    const unsigned t = next_tile;
-    __syncthreads();
-    if (t >= a.ntiles) break;
-    adjoint_tile(a, g, spiral, slot_mem, flags, stats, (int)(t % a.tiles_x),
-                 (int)(t / a.tiles_x));
-  }
+  atomicAdd(&stats[3], (unsigned long long)ws.cells);
+  atomicAdd(&stats[4], (unsigned long long)ws.cands);
 }
 
 // dL/dln rho and dL/dln T in the original particle order.
@@ -411,29 +402,30 @@ cudaError_t adjoint_ray_launch(Context& c, const RenderArgs& r, int mode, const 
   k.row0 = r.row0;
   k.row_end = r.rows > 0 ? (r.row0 + r.rows < r.ny ? r.row0 + r.rows : r.ny) : r.ny;
   const GridView g = make_grid_view(c);
-  dim3 grid((r.nx + 15) / 16, (k.row_end - k.row0 + 7) / 8);
-  k.queue = nullptr;
-  k.tiles_x = grid.x;
-  k.ntiles = grid.x * grid.y;
-  {
-    int sms = 0, per_sm = 0;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c.device);
-    const cudaError_t oe =
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, adjoint_kernel, 128, 0);
-    const unsigned resident = (unsigned)((sms > 0 ? sms : 148) * (per_sm > 0 ? per_sm : 1));
-    if (oe == cudaSuccess && k.ntiles > resident) {
-      if ((e = c.tile_queue.ensure(256))) return e;
-      if ((e = cudaMemsetAsync(c.tile_queue.p, 0, 4, c.stream))) return e;
-      k.queue = c.tile_queue.as<unsigned>();
-      grid = dim3(resident, 1);
-    }
-  }
+  k.tiles_x = (unsigned)((r.nx + 15) / 16);
+  const unsigned long long tiles =
+      (unsigned long long)k.tiles_x * (unsigned)((k.row_end - k.row0 + 7) / 8);
+  k.n_rays = 128ull * tiles;
+  if ((e = c.tile_queue.ensure(256))) return e;
+  if ((e = cudaMemsetAsync(c.tile_queue.p, 0, 8, c.stream))) return e;
+  k.queue = c.tile_queue.as<unsigned long long>();
+  int sms = 0, per_sm = 0;
+  if ((e = cudaFuncSetAttribute(adjoint_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)sizeof(AdjMem))) ||
+      (e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c.device)) ||
+      (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, adjoint_kernel, kListThreads,
+                                                         sizeof(AdjMem))))
+    return e;
+  const unsigned long long resident = (unsigned long long)sms * (per_sm > 0 ? per_sm : 1);
+  const unsigned blocks = (unsigned)(resident < 4 * tiles ? resident : 4 * tiles);
+  if ((e = c.list_over.ensure((size_t)blocks * kListWarps * kRays * kOver * 16))) return e;
+  k.over = c.list_over.as<float4>();
   if (!c.ev0) {
     if ((e = cudaEventCreate(&c.ev0)) || (e = cudaEventCreate(&c.ev1))) return e;
   }
   cudaEventRecord(c.ev0, c.stream);
   ++c.launches;
-  adjoint_kernel<<<grid, 128, 0, c.stream>>>(
+  adjoint_kernel<<<blocks, kListThreads, sizeof(AdjMem), c.stream>>>(
       k, g, c.spiral.as<char4>(), c.flags.as<uint32_t>(),
       reinterpret_cast<unsigned long long*>(c.flags.as<char>() + 64));
   if ((e = cudaGetLastError())) return e;

@@ -24,16 +24,13 @@
 
 #include "ilc_device.cuh"
 #include "ilc_internal.h"
-#include "ilc_walk4.cuh"
+#include "ilc_raylist.cuh"
 
 namespace ilc {
 
 GridView make_grid_view(const Context& c);  // ilc_render.cu
 
 namespace {
-
-constexpr int kBThreads = 128;
-constexpr unsigned kFull = 0xffffffffu;
 
 struct BatchK {
   const JobDev* jobs;
@@ -46,10 +43,9 @@ struct BatchK {
   double atol, rtol;
   int64_t max_steps;
   int tile_w;
-  float window;
   const uint32_t* order;
   unsigned long long* queue;
-  int axis_z;       // every job looks along z (look x and y exactly 0)
+  float4* over;   // list overflow, kOver per resident ray
 };
 
 // Largest k with jobs[k].item_begin <= item.
@@ -105,44 +101,6 @@ __device__ __forceinline__ void ray_span(const JobDev& j, int ix, int iy, bool& 
   for (int i = 0; i < 3; ++i) o[i] = pix[i] + z0f * j.look[i];
 }
 
-// Weights of point J's slots (get_weight3d) and their sum, in slot order.
-template <int J>
-__device__ __forceinline__ void slot_weights(const Step4& s, float w[8], float& ws) {
-#pragma unroll
-  for (int t = 0; t < 8; ++t) w[t] = weight3d(s4_d(s, J, t));
-  ws = 0.0f;
-#pragma unroll
-  for (int t = 0; t < 8; ++t) ws = ws + w[t];
-}
-
-// Single-channel value of point J (nn8 finalize order), from the channel
-// table or, without one, from the particles' q.
-template <int J>
-__device__ __forceinline__ float value1(const Step4& s, const float* __restrict__ chan,
-                                        const float4* __restrict__ parts) {
-  float w[8], ws;
-  slot_weights<J>(s, w, ws);
-  float dot = 0.0f;
-#pragma unroll
-  for (int t = 0; t < 8; ++t) {
-    const int id = __float_as_int(s4_v(s, J, t));
-    const float v = id < 0 ? 0.0f : (chan ? __ldg(&chan[id]) : __ldg(&parts[id].w));
-    dot = __fmaf_rn(w[t], v, dot);
-  }
-  return (ws != 0.0f && dot != 0.0f) ? dot / ws : 0.0f;
-}
-
-// Hands point J's slots to the warp: the distances become weights in place
-// (the indices stay), and their sum goes to wsum.
-template <int J>
-__device__ __forceinline__ void slots_to_weights(const Step4& s, float& wsum) {
-  float w[8], ws;
-  slot_weights<J>(s, w, ws);
-#pragma unroll
-  for (int t = 0; t < 8; ++t) s4_d(s, J, t) = w[t];
-  wsum = ws;
-}
-
 // One channel's FP64 step candidate: returns I + delta4 (as the accepted
 // value) and sets x to the channel's error ratio
 // max(atol, |I/z' rtol|) h / (2 |delta5 - delta4|), or 16 if delta4 == delta5.
@@ -165,258 +123,296 @@ __device__ __forceinline__ float channel_step(float Ic, float k1c, float e0, flo
   return (float)((double)Ic + d4);
 }
 
-// kMulti: V > 1 channels from the table. kOwnVal (V = 1 without a channel
-// table): the slots carry the particles' own q, as the render kernel's walk
-// does, so no value is looked up by index afterwards.
-template <bool kMulti, int kMinBlocks, bool kOwnVal, bool kAxis = false>
-__global__ void __launch_bounds__(kBThreads, kMinBlocks)
-batched_kernel(BatchK a, GridView g, const char4* __restrict__ spiral_g,
-               uint32_t* __restrict__ flags, unsigned long long* __restrict__ stats) {
-  __shared__ char4 spiral[1000];
-  // slot arrays of the walks; for V > 1 also the hand-over to the warp:
-  // weights in the distance rows, indices in the value rows, sums in slot_ws
-  __shared__ SlotMem slot_mem;
-  __shared__ float slot_ws[kMulti ? 4 : 1][kBThreads];
+// V > 1: the hand-over of a step's slots from the points' lanes to the warp.
+struct ChanHand {
+  float w[32][kRays];   // row 8 j + t: weight of slot t of point j
+  int id[32][kRays];    // its sorted particle index (-1: empty)
+  float ws[4][kRays];   // sum of point j's weights
+};
+
+template <bool kMulti> struct BlockMem {
+  char4 spiral[1000];
+  WarpLists lists[kListWarps];
+  ChanHand hand[kMulti ? kListWarps : 1];
   // the block's work counters (steps, accepted, -, cells, candidates, max
-  // steps of a ray, rays at the step limit), added per tile: kept out of the
-  // registers the walk needs
-  __shared__ unsigned long long blk_stats[7];
-  if (threadIdx.x < 7) blk_stats[threadIdx.x] = 0ull;
-  load_spiral(spiral, spiral_g);
+  // steps of a ray, rays at the step limit)
+  unsigned long long stats[7];
+};
+
+// kMulti: V > 1 channels from the table; the slots carry sorted indices.
+// Otherwise they carry the values (V = 1: the table's, or the particles' own
+// q). Every group of 4 lanes takes the next
+// ray of the queue when its ray has ended, so a warp's 8 rays need not be of
+// one length. Bound by instruction issue of the list replays (DRAM idle, the
+// grid sits in L2).
+template <bool kMulti, int kMinBlocks>
+__global__ void __launch_bounds__(kListThreads, kMinBlocks)
+batched_kernel(const __grid_constant__ BatchK a, const __grid_constant__ GridView g,
+               const char4* __restrict__ spiral_g, uint32_t* __restrict__ flags,
+               unsigned long long* __restrict__ stats) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  BlockMem<kMulti>& M = *reinterpret_cast<BlockMem<kMulti>*>(smem_raw);
+  if (threadIdx.x < 7) M.stats[threadIdx.x] = 0ull;
+  load_spiral(M.spiral, spiral_g);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int r = lane >> 2, pj = lane & 3;
+  WarpLists& W = M.lists[warp];
+  const unsigned wg = blockIdx.x * kListWarps + warp;
+  if (lane == 0) W.over = a.over + (size_t)wg * kRays * kOver;
+  ChanHand& H = M.hand[kMulti ? warp : 0];
   const int tw = a.tile_w, th = a.tile_w > 0 ? 32 / a.tile_w : 1;
-  float* wstate = kMulti ? a.state + ((size_t)blockIdx.x * kBThreads + (size_t)warp * 32) *
-                                         4 * (size_t)a.V
+  float* wstate = kMulti ? a.state + ((size_t)blockIdx.x * kListThreads / 4 +
+                                      (size_t)warp * kRays) * 4 * (size_t)a.V
                          : nullptr;
+  const float ext0 = 0.06f * g.cs0;
+  const unsigned long long n_rays = 32ull * a.n_items;
+  // this group's ray
+  bool have = false, drained = false, fresh = true;
+  float ox = 0.0f, oy = 0.0f, oz = 0.0f, lx = 0.0f, ly = 0.0f, lz = 0.0f, len = 0.0f;
+  float z = 0.0f, h = 1.0f, I = 0.0f, k1 = 0.0f, scale = 0.0f;
+  size_t out = 0, plane = 0;
+  uint32_t rs = 0, ra = 0;
+  WalkStats ws;
   for (;;) {
-    unsigned long long item = 0;
-    if (lane == 0) item = atomicAdd(a.queue, 1ull);
-    item = __shfl_sync(kFull, item, 0);
-    if (item >= a.n_items) break;
-    if (a.order) item = a.order[item];
-    const JobDev& J = a.jobs[find_job(a.jobs, a.n_jobs, item)];
-    const uint64_t t = item - J.item_begin;
-    int ix, iy;
-    bool inside;
-    if (tw > 0) {  // compact tile of tw x th pixels
-      const int tx = (int)(t % (uint64_t)J.tiles_x), ty = (int)(t / (uint64_t)J.tiles_x);
-      ix = tx * tw + lane % tw;
-      iy = ty * th + lane / tw;
-      inside = ix < J.nx && iy < J.ny;
-    } else {       // strided: pixels t, t + T, t + 2T, ... (T = items of the job)
-      const uint64_t pix = t + (uint64_t)lane * (uint64_t)J.tiles_x;
-      inside = pix < (uint64_t)J.nx * (uint64_t)J.ny;
-      ix = inside ? (int)(pix % (uint64_t)J.nx) : J.nx;
-      iy = inside ? (int)(pix / (uint64_t)J.nx) : J.ny;
-    }
-    bool masked = true;
-    float o[3] = {0.0f, 0.0f, 0.0f}, len = 0.0f;
-    if (inside) ray_span(J, ix, iy, masked, o, len);
-    const float lx = J.look[0], ly = J.look[1], lz = J.look[2];
-    bool run = inside && !masked;
-    float z = 0.0f, h = 1.0f, I = 0.0f, k1 = 0.0f;
-    float pts[4];
-    rkf_points(0.0f, 1.0f, pts);
-    uint32_t rs = 0, ra = 0;
-    WalkStats ws;
-    if (kMulti) {
-      for (int i = lane; i < 32 * 4 * a.V; i += 32) wstate[i] = 0.0f;
-      __syncwarp();
-    }
-    // z windows: the rays of the warp step up to the window's end, then the
-    // warp moves on together, so its 32 rays query one slab of the grid at a
-    // time. This orders the work only; each ray's steps are unchanged.
-    float wend = a.window > 0.0f ? a.window : FLT_MAX;
-    while (__any_sync(kFull, run && z < len)) {
-      if (!__any_sync(kFull, run && z < len && z < wend)) {
-        wend += a.window;
-        continue;
-      }
-      if (run && z < len && z < wend && (int64_t)rs >= a.max_steps) {
-        atomicAdd(&blk_stats[6], 1ull);
-        run = false;
-      }
-      const bool go = run && z < len && z < wend;
-      if (go) {
-        Step4 s;
-        s4_bind(s, slot_mem);
-        nn8_walk_step4<!kOwnVal, kAxis>(g, spiral, o[0], o[1], o[2], lx, ly, lz, pts, s, ws);
-        if (!kMulti) {
-          float e[4];
-          if (kOwnVal) {
-            e[0] = s4_finalize<0>(s);
-            e[1] = s4_finalize<1>(s);
-            e[2] = s4_finalize<2>(s);
-            e[3] = s4_finalize<3>(s);
-          } else {
-            e[0] = value1<0>(s, a.chan, g.parts);
-            e[1] = value1<1>(s, a.chan, g.parts);
-            e[2] = value1<2>(s, a.chan, g.parts);
-            e[3] = value1<3>(s, a.chan, g.parts);
-          }
-          const float zb = z;
-          rkf_advance_fp64(I, z, h, k1, a.atol, a.rtol, len, e, kEps, kHmin, kHmax, pts);
-          ++rs;
-          if (z != zb) ++ra;
+    // groups without a ray take the next ones
+    for (;;) {
+      const unsigned want = __ballot_sync(kAll, !have && !drained && pj == 0);
+      if (!want) break;
+      const unsigned long long q = take_rays(a.queue, want, fresh, lane, wg);
+      fresh = false;
+      if (!have && !drained) {
+        if (q >= n_rays) {
+          drained = true;
         } else {
-          slots_to_weights<0>(s, slot_ws[0][threadIdx.x]);
-          slots_to_weights<1>(s, slot_ws[1][threadIdx.x]);
-          slots_to_weights<2>(s, slot_ws[2][threadIdx.x]);
-          slots_to_weights<3>(s, slot_ws[3][threadIdx.x]);
-        }
-      }
-      if (kMulti) {
-        __syncwarp();
-        unsigned gom = __ballot_sync(kFull, go);
-        bool my_acc = false;
-        double my_nh = 0.0;
-        while (gom) {
-          const int r = __ffs(gom) - 1;
-          gom &= gom - 1;
-          const float zr = __shfl_sync(kFull, z, r), hr = __shfl_sync(kFull, h, r);
-          const int tr = warp * 32 + r;  // ray r's thread: its slot columns
-          float* Is = wstate + (size_t)r * 4 * a.V;
-          float* Ks = Is + a.V;
-          const double hd = (double)hr;
-          const float znew = zr + hr;
-          double xl = __longlong_as_double(0x7ff0000000000000ll);  // +inf
-          bool x0nan = false;
-          // candidate values (I + delta4, k5) go to the ray's scratch half
-          // and are committed once the warp knows the step is accepted
-          float* Es = Ks + a.V;
-          float* E2s = Es + a.V;
-          if ((a.V & 3) == 0) {
-            // rows of V = 4G floats: lane handles float4 groups lane, lane+32, ...
-            // (channels 4g..4g+3), one 16-byte load per neighbour and group
-            const int G = a.V >> 2;
-            const float4* __restrict__ chan4 = reinterpret_cast<const float4*>(a.chan);
-#pragma unroll 1
-            for (int gi = lane; gi < G; gi += 32) {
-              float ev[4][4];
-#pragma unroll
-              for (int p = 0; p < 4; ++p) {
-                float dot[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll
-                for (int q = 0; q < 8; ++q) {
-                  const int id = __float_as_int(slot_mem.v[p * 8 + q][tr]);
-                  const float4 v = id >= 0 ? __ldg(&chan4[(size_t)id * G + gi])
-                                           : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                  const float wq = slot_mem.d[p * 8 + q][tr];
-                  dot[0] = __fmaf_rn(wq, v.x, dot[0]);
-                  dot[1] = __fmaf_rn(wq, v.y, dot[1]);
-                  dot[2] = __fmaf_rn(wq, v.z, dot[2]);
-                  dot[3] = __fmaf_rn(wq, v.w, dot[3]);
-                }
-                const float wsum = slot_ws[p][tr];
-#pragma unroll
-                for (int k = 0; k < 4; ++k)
-                  ev[p][k] = (wsum != 0.0f && dot[k] != 0.0f) ? dot[k] / wsum : 0.0f;
-              }
-#pragma unroll
-              for (int k = 0; k < 4; ++k) {
-                const int c = 4 * gi + k;
-                double x;
-                Es[c] = channel_step(Is[c], Ks[c], ev[0][k], ev[1][k], ev[2][k], ev[3][k], hd,
-                                     znew, a.atol, a.rtol, x);
-                E2s[c] = ev[2][k];
-                if (c == 0 && isnan(x)) x0nan = true;
-                xl = fmin(xl, x);
+          const unsigned long long qi = q >> 5;
+          const int ti = (int)(q & 31);
+          const uint64_t item = a.order ? (uint64_t)a.order[qi] : qi;
+          const JobDev& J = a.jobs[find_job(a.jobs, a.n_jobs, item)];
+          const uint64_t t = item - J.item_begin;
+          int ix, iy;
+          bool inside;
+          if (tw > 0) {  // compact tile of tw x th pixels
+            const int tx = (int)(t % (uint64_t)J.tiles_x), ty = (int)(t / (uint64_t)J.tiles_x);
+            ix = tx * tw + ti % tw;
+            iy = ty * th + ti / tw;
+            inside = ix < J.nx && iy < J.ny;
+          } else {       // strided: pixels t, t + T, t + 2T, ... (T = items of the job)
+            const uint64_t pix = t + (uint64_t)ti * (uint64_t)J.tiles_x;
+            inside = pix < (uint64_t)J.nx * (uint64_t)J.ny;
+            ix = inside ? (int)(pix % (uint64_t)J.nx) : J.nx;
+            iy = inside ? (int)(pix / (uint64_t)J.nx) : J.ny;
+          }
+          if (inside) {
+            bool masked;
+            float o[3];
+            ray_span(J, ix, iy, masked, o, len);
+            plane = (size_t)J.nx * (size_t)J.ny;
+            out = J.out_offset + (size_t)iy * J.nx + ix;
+            if (masked || !(0.0f < len)) {  // no step: the pixel is 0
+              const float v = masked ? 0.0f : 0.0f * J.scale;
+              for (int c = pj; c < a.V; c += 4) a.out[out + (size_t)c * plane] = v;
+            } else {
+              have = true;
+              ox = o[0];
+              oy = o[1];
+              oz = o[2];
+              lx = J.look[0];
+              ly = J.look[1];
+              lz = J.look[2];
+              scale = J.scale;
+              z = 0.0f;
+              h = 1.0f;
+              I = 0.0f;
+              k1 = 0.0f;
+              rs = 0;
+              ra = 0;
+              if (pj == 0) ray_reset(W.meta[r], ext0);
+              if (kMulti) {
+                float* st = wstate + (size_t)r * 4 * a.V;
+                for (int c = pj; c < 4 * a.V; c += 4) st[c] = 0.0f;
               }
             }
-          } else {
+          }
+        }
+      }
+      __syncwarp();
+    }
+    if (!__any_sync(kAll, have)) break;
+    const float zq = step_point(z, h, pj);
+    PointSlots s;
+    bool go = have;
+    if (go && (int64_t)rs >= a.max_steps) {
+      if (pj == 0) atomicAdd(&M.stats[6], 1ull);
+      go = false;
+    }
+    eval_points<kMulti>(g, M.spiral, W, lane, go, ox, oy, oz, lx, ly, lz, zq, s, ws);
+    if (!kMulti) {
+      float e[4];
+      share4(go ? slots_value(s) : 0.0f, lane, e);
+      if (go) {
+        const float zb = z;
+        float next[4];
+        rkf_advance_fp64(I, z, h, k1, a.atol, a.rtol, len, e, kEps, kHmin, kHmax, next);
+        ++rs;
+        if (z != zb) ++ra;
+      }
+    } else {
+      if (go) {
+        float w[8], sum;
+        slot_weights(s, w, sum);
+#pragma unroll
+        for (int t = 0; t < 8; ++t) {
+          H.w[8 * pj + t][r] = w[t];
+          H.id[8 * pj + t][r] = __float_as_int(s.v[t]);
+        }
+        H.ws[pj][r] = sum;
+      }
+      __syncwarp();
+      unsigned gom = __ballot_sync(kAll, go && pj == 0);
+      bool my_acc = false;
+      double my_nh = 0.0;
+      while (gom) {
+        const int gl = __ffs(gom) - 1, tr = gl >> 2;
+        gom &= gom - 1;
+        const float zr = __shfl_sync(kAll, z, gl), hr = __shfl_sync(kAll, h, gl);
+        float* Is = wstate + (size_t)tr * 4 * a.V;
+        float* Ks = Is + a.V;
+        const double hd = (double)hr;
+        const float znew = zr + hr;
+        double xl = __longlong_as_double(0x7ff0000000000000ll);  // +inf
+        bool x0nan = false;
+        // candidate values (I + delta4, k5) go to the ray's scratch half
+        // and are committed once the warp knows the step is accepted
+        float* Es = Ks + a.V;
+        float* E2s = Es + a.V;
+        if ((a.V & 3) == 0) {
+          // rows of V = 4G floats: lane handles float4 groups lane, lane+32, ...
+          // (channels 4g..4g+3), one 16-byte load per neighbour and group
+          const int G = a.V >> 2;
+          const float4* __restrict__ chan4 = reinterpret_cast<const float4*>(a.chan);
 #pragma unroll 1
-            for (int c = lane; c < a.V; c += 32) {
-              float ev[4];
+          for (int gi = lane; gi < G; gi += 32) {
+            float ev[4][4];
 #pragma unroll
-              for (int p = 0; p < 4; ++p) {
-                float dot = 0.0f;
+            for (int p = 0; p < 4; ++p) {
+              float dot[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
-                for (int q = 0; q < 8; ++q) {
-                  const int id = __float_as_int(slot_mem.v[p * 8 + q][tr]);
-                  const float v = id >= 0 ? __ldg(&a.chan[(size_t)id * a.V + c]) : 0.0f;
-                  dot = __fmaf_rn(slot_mem.d[p * 8 + q][tr], v, dot);
-                }
-                const float wsum = slot_ws[p][tr];
-                ev[p] = (wsum != 0.0f && dot != 0.0f) ? dot / wsum : 0.0f;
+              for (int q = 0; q < 8; ++q) {
+                const int id = H.id[p * 8 + q][tr];
+                const float4 v = id >= 0 ? __ldg(&chan4[(size_t)id * G + gi])
+                                         : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                const float wq = H.w[p * 8 + q][tr];
+                dot[0] = __fmaf_rn(wq, v.x, dot[0]);
+                dot[1] = __fmaf_rn(wq, v.y, dot[1]);
+                dot[2] = __fmaf_rn(wq, v.z, dot[2]);
+                dot[3] = __fmaf_rn(wq, v.w, dot[3]);
               }
+              const float wsum = H.ws[p][tr];
+#pragma unroll
+              for (int k = 0; k < 4; ++k)
+                ev[p][k] = (wsum != 0.0f && dot[k] != 0.0f) ? dot[k] / wsum : 0.0f;
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              const int c = 4 * gi + k;
               double x;
-              Es[c] = channel_step(Is[c], Ks[c], ev[0], ev[1], ev[2], ev[3], hd, znew, a.atol,
-                                   a.rtol, x);
-              E2s[c] = ev[2];
+              Es[c] = channel_step(Is[c], Ks[c], ev[0][k], ev[1][k], ev[2][k], ev[3][k], hd, znew,
+                                   a.atol, a.rtol, x);
+              E2s[c] = ev[2][k];
               if (c == 0 && isnan(x)) x0nan = true;
               xl = fmin(xl, x);
             }
           }
-#pragma unroll
-          for (int off = 16; off > 0; off >>= 1) xl = fmin(xl, __shfl_xor_sync(kFull, xl, off));
-          // The host-side definition takes x_0 and then every smaller x_c:
-          // a NaN x_0 gives NaN, any other NaN is passed over.
-          const bool n0 = __shfl_sync(kFull, x0nan, 0);
-          const double xmin = n0 ? __longlong_as_double(0x7ff8000000000000ll) : xl;
-          double sc = sqrt(sqrt(xmin));
-          double nh = sc * hd;
-          if (nh < (double)kHmin) nh = (double)kHmin;
-          else if (nh > (double)kHmax) nh = (double)kHmax;
-          sc = nh / hd;
-          const bool accept = !(sc < 0.95);
-          if (accept) {
+        } else {
 #pragma unroll 1
-            for (int c = lane; c < a.V; c += 32) {
-              Is[c] = Es[c];
-              Ks[c] = E2s[c];
+          for (int c = lane; c < a.V; c += 32) {
+            float ev[4];
+#pragma unroll
+            for (int p = 0; p < 4; ++p) {
+              float dot = 0.0f;
+#pragma unroll
+              for (int q = 0; q < 8; ++q) {
+                const int id = H.id[p * 8 + q][tr];
+                const float v = id >= 0 ? __ldg(&a.chan[(size_t)id * a.V + c]) : 0.0f;
+                dot = __fmaf_rn(H.w[p * 8 + q][tr], v, dot);
+              }
+              const float wsum = H.ws[p][tr];
+              ev[p] = (wsum != 0.0f && dot != 0.0f) ? dot / wsum : 0.0f;
             }
-          }
-          if (lane == r) {
-            my_acc = accept;
-            my_nh = nh;
+            double x;
+            Es[c] = channel_step(Is[c], Ks[c], ev[0], ev[1], ev[2], ev[3], hd, znew, a.atol,
+                                 a.rtol, x);
+            E2s[c] = ev[2];
+            if (c == 0 && isnan(x)) x0nan = true;
+            xl = fmin(xl, x);
           }
         }
-        __syncwarp();
-        if (go) {
-          const float znew = z + h;
-          if (my_acc) z = znew;
-          h = (float)my_nh;
-          if (z + h >= len) h = len - z + kEps;
-          rkf_points(z, h, pts);
-          ++rs;
-          if (my_acc) ++ra;
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) xl = fmin(xl, __shfl_xor_sync(kAll, xl, off));
+        // The host-side definition takes x_0 and then every smaller x_c:
+        // a NaN x_0 gives NaN, any other NaN is passed over.
+        const bool n0 = __shfl_sync(kAll, x0nan, 0);
+        const double xmin = n0 ? __longlong_as_double(0x7ff8000000000000ll) : xl;
+        double sc = sqrt(sqrt(xmin));
+        double nh = sc * hd;
+        if (nh < (double)kHmin) nh = (double)kHmin;
+        else if (nh > (double)kHmax) nh = (double)kHmax;
+        sc = nh / hd;
+        const bool accept = !(sc < 0.95);
+        if (accept) {
+#pragma unroll 1
+          for (int c = lane; c < a.V; c += 32) {
+            Is[c] = Es[c];
+            Ks[c] = E2s[c];
+          }
+        }
+        if (r == tr) {
+          my_acc = accept;
+          my_nh = nh;
         }
       }
-    }
-    // outputs of the tile
-    if (!kMulti) {
-      if (inside)
-        a.out[J.out_offset + (size_t)iy * J.nx + ix] = masked ? 0.0f : I * J.scale;
-    } else {
       __syncwarp();
-      const size_t plane = (size_t)J.nx * (size_t)J.ny;
-      for (int r = 0; r < 32; ++r) {
-        const int ixr = __shfl_sync(kFull, ix, r), iyr = __shfl_sync(kFull, iy, r);
-        const bool in_r = __shfl_sync(kFull, inside, r), m_r = __shfl_sync(kFull, masked, r);
-        if (!in_r) continue;
+      if (go) {
+        const float znew = z + h;
+        if (my_acc) z = znew;
+        h = (float)my_nh;
+        if (z + h >= len) h = len - z + kEps;
+        ++rs;
+        if (my_acc) ++ra;
+      }
+    }
+    // rays that ended (or reached the step limit)
+    const bool fin = have && (!go || !(z < len));
+    if (fin) {
+      if (kMulti) {
         const float* Is = wstate + (size_t)r * 4 * a.V;
-        for (int c = lane; c < a.V; c += 32)
-          a.out[J.out_offset + (size_t)c * plane + (size_t)iyr * J.nx + ixr] =
-              m_r ? 0.0f : Is[c] * J.scale;
+        for (int c = pj; c < a.V; c += 4) a.out[out + (size_t)c * plane] = Is[c] * scale;
+      } else if (pj == 0) {
+        a.out[out] = I * scale;
       }
-      __syncwarp();
+      if (pj == 0) {
+        atomicAdd(&M.stats[0], (unsigned long long)rs);
+        atomicAdd(&M.stats[1], (unsigned long long)ra);
+        atomicMax(&M.stats[5], (unsigned long long)rs);
+      }
+      atomicAdd(&M.stats[3], (unsigned long long)ws.cells);
+      atomicAdd(&M.stats[4], (unsigned long long)ws.cands);
+      ws.cells = 0;
+      ws.cands = 0;
+      have = false;
     }
-    atomicAdd(&blk_stats[0], (unsigned long long)rs);
-    atomicAdd(&blk_stats[1], (unsigned long long)ra);
-    atomicAdd(&blk_stats[3], (unsigned long long)ws.cells);
-    atomicAdd(&blk_stats[4], (unsigned long long)ws.cands);
-    atomicMax(&blk_stats[5], (unsigned long long)rs);
+    __syncwarp();
   }
   __syncthreads();
   if (threadIdx.x == 0) {
-    if (blk_stats[6]) atomicOr(flags, FLAG_STEP_LIMIT);
-    atomicAdd(&stats[0], blk_stats[0]);
-    atomicAdd(&stats[1], blk_stats[1]);
-    atomicAdd(&stats[2], 4ull * blk_stats[0]);
-    atomicAdd(&stats[3], blk_stats[3]);
-    atomicAdd(&stats[4], blk_stats[4]);
-    atomicMax(&stats[5], blk_stats[5]);
-    atomicAdd(&stats[6], blk_stats[6]);
+    if (M.stats[6]) atomicOr(flags, FLAG_STEP_LIMIT);
+    atomicAdd(&stats[0], M.stats[0]);
+    atomicAdd(&stats[1], M.stats[1]);
+    atomicAdd(&stats[2], 4ull * M.stats[0]);
+    atomicAdd(&stats[3], M.stats[3]);
+    atomicAdd(&stats[4], M.stats[4]);
+    atomicMax(&stats[5], M.stats[5]);
+    atomicAdd(&stats[6], M.stats[6]);
   }
 }
 
@@ -456,62 +452,46 @@ __global__ void tile_cost_kernel(const float4* __restrict__ parts,
   }
 }
 
-template <bool kMulti, int kMinBlocks>
-int persistent_blocks(const Context& c) {
+// One channel: 4 blocks of 128 threads per SM (126 registers, 54 KB of shared
+// memory); V > 1 adds the hand-over and runs 3.
+template <bool kMulti> struct Variant {
+  static constexpr int kBlocks = kMulti ? 3 : 4;
+  static constexpr size_t kSmem = sizeof(BlockMem<kMulti>);
+  static auto kernel() { return batched_kernel<kMulti, kBlocks>; }
+};
+
+// Resident blocks: what registers and shared memory allow, or `occ` per SM.
+template <bool kMulti> cudaError_t persistent_blocks(const Context& c, int occ, int* blocks) {
+  using Vt = Variant<kMulti>;
   int sms = 0, per_sm = 0;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c.device);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm,
-                                                batched_kernel<kMulti, kMinBlocks, false>,
-                                                kBThreads, 0);
-  if (sms <= 0) sms = 148;
-  if (per_sm <= 0) per_sm = 1;
-  return sms * per_sm;
+  cudaError_t e;
+  if ((e = cudaFuncSetAttribute(Vt::kernel(), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)Vt::kSmem)))
+    return e;
+  if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c.device))) return e;
+  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, Vt::kernel(), kListThreads,
+                                                         Vt::kSmem)))
+    return e;
+  if (occ > 0) per_sm = std::min(per_sm, occ);
+  *blocks = sms * std::max(per_sm, 1);
+  return cudaSuccess;
 }
 
-template <bool kMulti, int kMinBlocks>
+template <bool kMulti>
 cudaError_t launch_variant(Context& c, const BatchK& k, const GridView& g, int blocks) {
+  using Vt = Variant<kMulti>;
   unsigned long long* stats = reinterpret_cast<unsigned long long*>(c.flags.as<char>() + 64);
-  if constexpr (!kMulti) {
-    if (!k.chan) {
-      if (k.axis_z)
-        batched_kernel<false, kMinBlocks, true, true><<<blocks, kBThreads, 0, c.stream>>>(
-            k, g, c.spiral.as<char4>(), c.flags.as<uint32_t>(), stats);
-      else
-        batched_kernel<false, kMinBlocks, true><<<blocks, kBThreads, 0, c.stream>>>(
-            k, g, c.spiral.as<char4>(), c.flags.as<uint32_t>(), stats);
-      return cudaGetLastError();
-    }
-  }
-  batched_kernel<kMulti, kMinBlocks, false><<<blocks, kBThreads, 0, c.stream>>>(
-      k, g, c.spiral.as<char4>(), c.flags.as<uint32_t>(), stats);
+  Vt::kernel()<<<blocks, kListThreads, Vt::kSmem, c.stream>>>(k, g, c.spiral.as<char4>(),
+                                                              c.flags.as<uint32_t>(), stats);
   return cudaGetLastError();
 }
 
-int variant_blocks(const Context& c, bool multi, int occ) {
-  if (multi)
-    return occ == 5   ? persistent_blocks<true, 5>(c)
-           : occ == 4 ? persistent_blocks<true, 4>(c)
-           : occ == 3 ? persistent_blocks<true, 3>(c)
-                      : persistent_blocks<true, 1>(c);
-  return occ == 5   ? persistent_blocks<false, 5>(c)
-         : occ == 4 ? persistent_blocks<false, 4>(c)
-         : occ == 3 ? persistent_blocks<false, 3>(c)
-                    : persistent_blocks<false, 1>(c);
-}
-
-cudaError_t enqueue(Context& c, const BatchK& k, const GridView& g, int occ, int blocks) {
+cudaError_t enqueue(Context& c, const BatchK& k, const GridView& g, int blocks) {
   cudaError_t e;
   if ((e = cudaMemsetAsync(c.flags.p, 0, kFlagsBytes, c.stream))) return e;
   if ((e = cudaMemsetAsync(c.queue.p, 0, 8, c.stream))) return e;
-  if (k.V == 1)
-    return occ == 5   ? launch_variant<false, 5>(c, k, g, blocks)
-           : occ == 4 ? launch_variant<false, 4>(c, k, g, blocks)
-           : occ == 3 ? launch_variant<false, 3>(c, k, g, blocks)
-                      : launch_variant<false, 1>(c, k, g, blocks);
-  return occ == 5   ? launch_variant<true, 5>(c, k, g, blocks)
-         : occ == 4 ? launch_variant<true, 4>(c, k, g, blocks)
-         : occ == 3 ? launch_variant<true, 3>(c, k, g, blocks)
-                    : launch_variant<true, 1>(c, k, g, blocks);
+  return k.V == 1 ? launch_variant<false>(c, k, g, blocks)
+                  : launch_variant<true>(c, k, g, blocks);
 }
 
 }  // namespace
@@ -576,23 +556,26 @@ cudaError_t batched_launch(Context& c, const BatchArgs& a, float* kernel_ms) {
   k.rtol = a.rtol;
   k.max_steps = c.max_steps;
   k.tile_w = a.tile_w;
-  k.window = a.window;
   k.order = a.order;
   k.queue = c.queue.as<unsigned long long>();
-  k.axis_z = a.axis_z ? 1 : 0;
-  const int occ = a.occupancy;
-  const int blocks = variant_blocks(c, a.V > 1, occ);
+  int blocks = 0;
+  if ((e = a.V > 1 ? persistent_blocks<true>(c, a.occupancy, &blocks)
+                   : persistent_blocks<false>(c, a.occupancy, &blocks)))
+    return e;
   if (a.V > 1) {
-    if ((e = c.chan_state.ensure((size_t)blocks * kBThreads * 4 * (size_t)k.V * 4))) return e;
+    if ((e = c.chan_state.ensure((size_t)blocks * (kListThreads / 4) * 4 * (size_t)k.V * 4)))
+      return e;
     k.state = c.chan_state.as<float>();
   }
-  const GridView g = make_grid_view(c);
+  if ((e = c.list_over.ensure((size_t)blocks * kListWarps * kRays * kOver * 16))) return e;
+  k.over = c.list_over.as<float4>();
+  GridView g = make_grid_view(c);
+  if (a.V == 1) g.vals = a.chan;
   if (!c.ev0) {
     if ((e = cudaEventCreate(&c.ev0)) || (e = cudaEventCreate(&c.ev1))) return e;
   }
   std::string key(reinterpret_cast<const char*>(&k), sizeof(k));
   key.append(reinterpret_cast<const char*>(&g), sizeof(g));
-  key.append(reinterpret_cast<const char*>(&occ), sizeof(occ));
   key.append(reinterpret_cast<const char*>(&blocks), sizeof(blocks));
   if (!c.batch_exec || key != c.batch_key) {
     if (c.batch_exec) {
@@ -602,7 +585,7 @@ cudaError_t batched_launch(Context& c, const BatchArgs& a, float* kernel_ms) {
     c.batch_key.clear();
     cudaGraph_t graph = nullptr;
     if ((e = cudaStreamBeginCapture(c.stream, cudaStreamCaptureModeThreadLocal))) return e;
-    const cudaError_t el = enqueue(c, k, g, occ, blocks);
+    const cudaError_t el = enqueue(c, k, g, blocks);
     e = cudaStreamEndCapture(c.stream, &graph);
     if (el) {
       if (graph) cudaGraphDestroy(graph);

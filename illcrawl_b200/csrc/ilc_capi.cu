@@ -274,11 +274,7 @@ ilc_status batched_jobs(Context& c, int32_t V, const ilc_job* jobs, int32_t n_jo
   a->rtol = tol.relative;
   a->tile_w = c.batch_tile_w;
   a->occupancy = c.batch_occupancy;
-  a->window = c.batch_window;
   a->order = nullptr;
-  a->axis_z = true;
-  for (const JobDev& d : jd)
-    if (d.look[0] != 0.0f || d.look[1] != 0.0f) a->axis_z = false;
   if (c.batch_cost_order) ILC_CUDA(c, batched_order(c, *a, jd), "work order");
   return ILC_OK;
 }
@@ -487,7 +483,7 @@ void ilc_destroy(ilc_ctx* h) {
   Context& c = h->c;
   cudaSetDevice(c.device);
   if (c.stream) cudaStreamSynchronize(c.stream);
-  for (DevBuf* b : {&c.parts, &c.cells, &c.s2u, &c.keys_a, &c.keys_b, &c.vals_a, &c.vals_b,
+  for (DevBuf* b : {&c.tile_queue, &c.list_over, &c.parts, &c.cells, &c.s2u, &c.keys_a, &c.keys_b, &c.vals_a, &c.vals_b,
                     &c.hist, &c.tmp_in, &c.gaunt, &c.list_d, &c.list_v, &c.list_id, &c.in_a,
                     &c.in_b, &c.in_c, &c.out_a, &c.out_b, &c.out_c, &c.spiral, &c.flags,
                     &c.rec_h, &c.rec_n, &c.adj_dT, &c.adj_dR, &c.adj_grad, &c.adj_seed,
@@ -533,8 +529,7 @@ ilc_status ilc_set_z_window(ilc_ctx* h, float z_window) {
   if (!h) return ILC_ERR_INVALID_ARGUMENT;
   if (!(z_window >= 0.0f) || !std::isfinite(z_window))
     return fail(h->c, ILC_ERR_INVALID_ARGUMENT, "z_window must be finite and >= 0");
-  h->c.z_window = z_window;
-  return ILC_OK;
+  return ILC_OK;  // a hint without effect (see ilc.h)
 }
 
 ilc_status ilc_nn8_setup_particles(ilc_ctx* h, const float* particles, uint64_t n,
@@ -1285,7 +1280,6 @@ ilc_status ilc_autotune_render(ilc_ctx* h, const ilc_camera* cam, double z_range
     for (int32_t j = 0; j < n_occupancies; ++j) {
       if (occupancies[j] != 0 && occupancies[j] != 3 && occupancies[j] != 4 && occupancies[j] != 5)
         return fail(c, ILC_ERR_INVALID_ARGUMENT, "occupancy must be 0, 3, 4 or 5");
-      a.window_override = windows[i];
       a.occupancy_override = occupancies[j];
       float ms = 0.0f;
       ILC_CUDA(c, render_launch(c, a, &ms), "autotune render");
@@ -1303,7 +1297,6 @@ ilc_status ilc_autotune_render(ilc_ctx* h, const ilc_camera* cam, double z_range
       }
     }
   }
-  c.z_window = *best_window;
   c.render_occupancy = *best_occupancy;
   return ILC_OK;
 }
@@ -1350,7 +1343,6 @@ ilc_status ilc_set_batch_schedule(ilc_ctx* h, int32_t tile_w, int32_t blocks_per
                 "tile_w 0 or 1..32 (powers of 2), occupancy 0, 3, 4 or 5, z_window >= 0");
   h->c.batch_tile_w = tile_w;
   h->c.batch_occupancy = blocks_per_sm;
-  h->c.batch_window = z_window;
   h->c.batch_cost_order = cost_order != 0;
   return ILC_OK;
 }
@@ -1421,12 +1413,10 @@ ilc_status ilc_autotune_batched(ilc_ctx* h, const float* values, int32_t n_chann
     len = std::max(len, e);
   }
   const int32_t keep_w = c.batch_tile_w, keep_o = c.batch_occupancy;
-  const float keep_z = c.batch_window;
   const bool keep_order = c.batch_cost_order;
   auto restore = [&]() {
     c.batch_tile_w = keep_w;
     c.batch_occupancy = keep_o;
-    c.batch_window = keep_z;
     c.batch_cost_order = keep_order;
   };
   float best = 0.0f;
@@ -1436,7 +1426,6 @@ ilc_status ilc_autotune_batched(ilc_ctx* h, const float* values, int32_t n_chann
       for (int32_t q = 0; q < n_windows; ++q) {
         c.batch_tile_w = tile_ws[i];
         c.batch_occupancy = occupancies[j];
-        c.batch_window = windows[q];
         c.batch_cost_order = true;
         BatchArgs a{};
         ilc_status st = batched_prepare(c, values, n_channels, values_on_device, jobs, n_jobs,
@@ -1472,7 +1461,6 @@ ilc_status ilc_autotune_batched(ilc_ctx* h, const float* values, int32_t n_chann
   }
   c.batch_tile_w = *best_tile_w;
   c.batch_occupancy = *best_occupancy;
-  c.batch_window = *best_window;
   c.batch_cost_order = true;
   return ILC_OK;
 }

@@ -322,13 +322,14 @@ __global__ void cell_ranges_kernel(const uint32_t* __restrict__ sk, uint64_t n,
   if (i + 1 == n || sk[i + 1] != k) cells[k].y = (int)(i + 1);
 }
 
-// Sub-box code of every sorted particle: which quarter of its cell it lies in
-// per axis (clamped to 0..3), packed sx + 4 sy + 16 sz. The nn8 walk uses it
-// only to skip candidates that lie, by more than a rounding margin, outside
-// the cube of the current search radius around the query points: those could
-// never be inserted, so skipping them leaves every result unchanged.
+// Sub-box code of every sorted particle: which sixteenth of its cell it lies in
+// per axis (clamped to 0..15), packed sx + 32 sy + 1024 sz (a free bit above
+// each field, for range tests by subtraction). The list builds use it only to
+// skip candidates that lie, by more than a rounding margin, outside the cube
+// of the current threshold around a point: those could never be inserted, so
+// skipping them leaves every result unchanged.
 __global__ void codes_kernel(const float4* __restrict__ parts, const uint32_t* __restrict__ sk,
-                             uint64_t n, KeyGrid kg, uint8_t* __restrict__ codes) {
+                             uint64_t n, KeyGrid kg, uint16_t* __restrict__ codes) {
   const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
   if (i >= n) return;
   const uint32_t k = sk[i];
@@ -338,14 +339,14 @@ __global__ void codes_kernel(const float4* __restrict__ parts, const uint32_t* _
   const float c[3] = {p.x, p.y, p.z};
   const float mn[3] = {kg.min0 + (float)kx * kg.cs0, kg.min1 + (float)ky * kg.cs1,
                        kg.min2 + (float)kz * kg.cs2};
-  const float iw[3] = {4.0f / kg.cs0, 4.0f / kg.cs1, 4.0f / kg.cs2};
+  const float iw[3] = {16.0f / kg.cs0, 16.0f / kg.cs1, 16.0f / kg.cs2};
   int q[3];
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
     const float t = (c[a] - mn[a]) * iw[a];
-    q[a] = t > 0.0f ? min((int)t, 3) : 0;
+    q[a] = t > 0.0f ? min((int)t, 15) : 0;
   }
-  codes[i] = (uint8_t)(q[0] | (q[1] << 2) | (q[2] << 4));
+  codes[i] = (uint16_t)(q[0] | (q[1] << 5) | (q[2] << 10));
 }
 
 inline unsigned grid_blocks(uint64_t n, int threads) {
@@ -394,7 +395,7 @@ cudaError_t grid_build_device(Context& c, const float4* in, uint64_t n) {
   if ((e = c.keys_a.ensure(n * 4)) || (e = c.keys_b.ensure(n * 4)) ||
       (e = c.vals_a.ensure(n * 4)) || (e = c.vals_b.ensure(n * 4)) ||
       (e = c.parts.ensure(n * 16)) || (e = c.s2u.ensure(n * 4)) ||
-      (e = c.codes.ensure(((n + 15) / 16) * 16 + 16)) || (e = c.cells.ensure(g.total * 8)) ||
+      (e = c.codes.ensure((n + 512) * 2)) || (e = c.cells.ensure(g.total * 8)) ||
       (e = c.flags.ensure(kFlagsBytes)))
     return e;
   const uint64_t tiles = (n + kSortTile - 1) / kSortTile;
@@ -429,7 +430,7 @@ cudaError_t grid_build_device(Context& c, const float4* in, uint64_t n) {
   if ((e = cudaMemsetAsync(c.cells.p, 0, g.total * 8, c.stream))) return e;
   cell_ranges_kernel<<<grid_blocks(n, 256), 256, 0, c.stream>>>(ka, n, c.cells.as<int2>());
   codes_kernel<<<grid_blocks(n, 256), 256, 0, c.stream>>>(c.parts.as<float4>(), ka, n, kg,
-                                                           c.codes.as<uint8_t>());
+                                                           c.codes.as<uint16_t>());
   c.launches += 4;  // keys, gather, cell ranges, codes
   return cudaGetLastError();
 }

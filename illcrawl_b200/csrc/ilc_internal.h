@@ -53,7 +53,6 @@ struct Context {
   int64_t max_steps = 1 << 20;  // per-ray RKF step cap
   uint64_t checkpoint_budget = 0;  // adjoint: device bytes for step checkpoints (0: a quarter
                                    // of the device's memory)
-  float z_window = 0.0f;        // adaptive render: z window of the block schedule (0 = none)
   int32_t render_occupancy = 4; // adaptive render: blocks per SM (0 = register-limited)
   int32_t render_engine = ILC_ENGINE_PERSISTENT;  // FP64 adaptive renders: kernel used
   int32_t query_engine = ILC_QUERY_THREAD;        // ilc_nn8_query: one thread or one warp per query
@@ -65,7 +64,7 @@ struct Context {
   DevBuf parts;      // float4 sorted particles
   DevBuf cells;      // int2 per grid cell
   DevBuf s2u;        // uint32 sorted -> original index
-  DevBuf codes;      // uint8 sub-box code per sorted particle (candidate pruning)
+  DevBuf codes;      // uint16 sub-box code per sorted particle (candidate pruning)
   const uint32_t* sorted_keys = nullptr;  // cell key per sorted particle (keys_a or keys_b)
   DevBuf keys_a, keys_b, vals_a, vals_b, hist, tmp_in;  // build scratch
 
@@ -87,7 +86,8 @@ struct Context {
 
   // generic per-call staging
   DevBuf in_a, in_b, in_c, out_a, out_b, out_c;
-  DevBuf tile_queue;  // persistent one-block-per-tile kernels: tile counter
+  DevBuf tile_queue;  // render and adjoint kernels: ray counter
+  DevBuf list_over;   // ray kernels: candidate lists beyond shared memory
   DevBuf spiral;     // char4[1000]
   DevBuf flags;      // uint32 error flags + uint64 stats
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -103,7 +103,6 @@ struct Context {
   DevBuf jobs, chan_sorted, chan_state, queue, item_cost, item_order;
   int32_t batch_tile_w = 8;       // batched work item: tile_w x (32 / tile_w) pixels
   int32_t batch_occupancy = 4;    // batched kernel: blocks per SM (0 = register-limited)
-  float batch_window = 40.0f;     // batched kernel: per-warp z window (0 = none)
   bool batch_cost_order = true;   // hand out the costliest tiles first
   cudaGraphExec_t batch_exec = nullptr;  // the batched launch sequence as a CUDA graph
   std::string batch_key;                 // launch parameters it was captured with
@@ -199,7 +198,6 @@ struct RenderArgs {
   bool apply_scale;
   float* out;           // device image
   double* out_d = nullptr;  // frozen replay: device image of the increments summed in double
-  float window_override = -1.0f;  // >= 0: z window for this launch (autotuner)
   int occupancy_override = -1;    // >= 0: occupancy variant for this launch (autotuner)
   int row_stride = 1;             // > 1: only every row_stride-th tile row (autotuner)
   float* rec_h = nullptr;         // adjoint checkpoint: accepted step sizes per ray
@@ -255,9 +253,7 @@ struct BatchArgs {
   double atol, rtol;
   int32_t tile_w;         // 1, 2, 4, 8, 16 or 32
   int32_t occupancy;      // 0, 3 or 4
-  float window;           // per-warp z window (0 = none)
   const uint32_t* order;  // device: work item handed out q-th (nullptr = natural order)
-  bool axis_z = false;    // every job looks along z (look x and y exactly 0)
 };
 // Estimated cost per work item of a batched render (the particles projected
 // into each tile's pixel columns, weighted by their cell's occupancy), and

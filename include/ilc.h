@@ -106,13 +106,13 @@ const char* ilc_last_error(const ilc_ctx* ctx);
 ilc_status ilc_set_step_limit(ilc_ctx* ctx, int64_t max_steps);
 /* The context's cudaStream_t, for callers that time or order work around it. */
 void* ilc_get_stream(ilc_ctx* ctx);
-/* Schedule of the adaptive render: rays of a thread block advance through
- * z_window-thick slabs together (0 = every ray runs to its end independently).
- * Changes the order of work only, never a result. */
+/* Schedule hint of the adaptive render (z window, >= 0), kept for callers that
+ * set it: the kernels carry each ray's candidates along the ray and let every
+ * ray run to its end on its own, so it changes neither results nor times. */
 ilc_status ilc_set_z_window(ilc_ctx* ctx, float z_window);
 /* Kernel behind ilc_render_adaptive and ilc_project_xray_flux with the FP64
- * controller. GRID: one thread block per 16 x 8 pixel tile, one launch per
- * image (the reference's one-projection-per-call structure). PERSISTENT: the
+ * controller. GRID: the rays of 16 x 8 pixel tiles in image order, one launch
+ * per image (the reference's one-projection-per-call structure). PERSISTENT: the
  * work-queue kernel of ilc_render_batched with this one camera (its
  * schedule: ilc_set_batch_schedule). Both give the same image bit for bit;
  * the REF32 controller, the fixed-step mode and the adjoint's forward pass
@@ -135,10 +135,9 @@ ilc_status ilc_set_query_engine(ilc_ctx* ctx, int32_t engine);
  * call that launches a kernel. No reference counterpart. */
 ilc_status ilc_nn8_query_stats(ilc_ctx* ctx, uint64_t* cells_visited, uint64_t* candidates);
 
-/* Occupancy of the adaptive render: 0 = as many blocks per SM as the
- * kernel's registers allow, 3, 4 or 5 = that many 128-thread blocks per SM
- * (registers capped accordingly). Changes the order of work only, never a
- * result. */
+/* Occupancy of the adaptive render: 0 = as many 128-thread blocks per SM as
+ * registers and shared memory allow, 3, 4 or 5 = at most that many. Changes
+ * the order of work only, never a result. */
 ilc_status ilc_set_render_occupancy(ilc_ctx* ctx, int32_t blocks_per_sm);
 
 /* ---- particle grid + nn8 backend ------------------------------------------
@@ -496,9 +495,9 @@ ilc_status ilc_render_batched(ilc_ctx* ctx, const float* values, int32_t n_chann
  * (32 / tile_w) pixels (tile_w in 1, 2, 4, 8, 16, 32), one per warp, or with
  * tile_w = 0 strided items (pixels k, k + T, k + 2T, ... of a job with T items,
  * which spreads the expensive rays of a small region over many warps); 0
- * (register-limited), 3, 4 or 5 blocks per SM; z_window > 0 makes a warp's rays
- * advance in windows of that depth (they query one slab of the grid at a
- * time); cost_order != 0 hands out the tiles in decreasing order of an
+ * (as many as fit), or at most 3, 4 or 5 blocks per SM; z_window >= 0 is
+ * accepted and has no effect (each ray runs to its end on its own);
+ * cost_order != 0 hands out the tiles in decreasing order of an
  * estimated cost (particles projected into each tile's columns, weighted by
  * their cell's occupancy), so the longest rays start first. Changes the order
  * of work only, never a result. Default: 8, 4, 40, 1. */
