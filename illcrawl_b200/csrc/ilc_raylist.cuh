@@ -65,7 +65,7 @@ constexpr unsigned kAll = 0xffffffffu;
 // how far the next list reaches.
 struct RayMeta {
   float za, zb, ext;
-  int n, nu;   // candidates before the first break cell; break cells
+  int n, nu, all;   // candidates before the first break cell; break cells; candidates
 };
 
 struct WarpLists {
@@ -193,59 +193,12 @@ __device__ __forceinline__ int warp_inclusive(int v, int lane) {
   return v;
 }
 
-// Candidates [p0, p1) of one cell, loaded 128 at a time. False: list overflow.
-template <bool kIdx>
-__device__ __forceinline__ bool take_range(const GridView& g, BuildState& b, WarpLists& W, int r,
-                                           int lane, float qx, float qy, float qz, int p0, int p1,
-                                           int k) {
-#pragma unroll 1
-  for (int p = p0; p < p1; p += 128) {
-    float4 P[4];
-    float d2[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int q = p + 32 * j + lane;
-      P[j] = __ldg(&g.parts[q < p1 ? q : p1 - 1]);
-    }
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float fx = P[j].x - qx, fy = P[j].y - qy, fz = P[j].z - qz;
-      d2[j] = (fx * fx + fy * fy) + fz * fz;
-    }
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int q = p + 32 * j + lane;
-      if (__any_sync(kAll, q < p1 && d2[j] < b.T2))
-        build_take<kIdx>(g, b, W, r, lane, q < p1, P[j], d2[j], q, k);
-    }
-    if (b.n > kCapAll) return false;
-  }
-  return true;
-}
-
-// The first n buffered hits, 32 at a time. False: list overflow.
-template <bool kIdx>
-__device__ __forceinline__ bool take_hits(const GridView& g, BuildState& b, WarpLists& W, int r,
-                                          int lane, float qx, float qy, float qz, int n, int k) {
-  __syncwarp();
-#pragma unroll 1
-  for (int h = 0; h < n; h += 32) {
-    const bool valid = h + lane < n;
-    const int p = W.hits[valid ? h + lane : h];
-    const float4 P = __ldg(&g.parts[p]);
-    const float fx = P.x - qx, fy = P.y - qy, fz = P.z - qz;
-    build_take<kIdx>(g, b, W, r, lane, valid, P, (fx * fx + fy * fy) + fz * fz, p, k);
-  }
-  __syncwarp();
-  return b.n <= kCapAll;
-}
-
 // Cells with more than kCodedMin candidates: the first kDirect are loaded (they
 // bring the radius down), the rest are read through their 2-byte sub-box
 // codes, 256 at a time, and only those whose sub-box meets the cube of the
 // threshold around the midpoint are loaded: a candidate outside it is farther
 // away than the threshold (which only shrinks).
-constexpr int kDirect = 128, kCodedMin = 384;
+constexpr int kDirect = 64, kCodedMin = 160;
 constexpr uint32_t kGuard = 0x42104210u;  // guard bits 4, 9, 14 of both codes
 
 // 4-bit field range [lo, hi] of [a, b] along one axis; false: none.
@@ -257,67 +210,25 @@ __device__ __forceinline__ bool code_range(float a, float b, float inv_w, uint32
   return th >= 0.0f && tl < 16.0f;
 }
 
-template <bool kIdx>
-__device__ __forceinline__ bool take_coded(const GridView& g, BuildState& b, WarpLists& W, int r,
-                                           int lane, float qx, float qy, float qz, float mx,
-                                           float my, float mz, int p0, int p1, int k) {
-  const uint4* __restrict__ codes = reinterpret_cast<const uint4*>(g.codes);  // 8 codes each
-  int nbuf = 0;
-  float used = -1.0f;
-  uint32_t lo = 0, hi = 0;
-  int pw = p0 & ~7;
-  uint4 nx = __ldg(codes + (pw >> 3) + lane);
-#pragma unroll 1
-  for (; pw < p1; pw += 256) {
-    const uint4 w4 = nx;
-    nx = __ldg(codes + ((pw + 256 < p1 ? pw + 256 : pw) >> 3) + lane);
-    if (b.T != used) {
-      used = b.T;
-      const float e = b.T + g.margin;
-      uint32_t l0, h0, l1, h1, l2, h2;
-      const bool in = code_range(qx - e - mx, qx + e - mx, g.inv_w0, l0, h0) &
-                      code_range(qy - e - my, qy + e - my, g.inv_w1, l1, h1) &
-                      code_range(qz - e - mz, qz + e - mz, g.inv_w2, l2, h2);
-      if (!in) break;  // no later candidate of the cell is within reach
-      lo = (l0 | (l1 << 5) | (l2 << 10)) * 0x10001u;
-      hi = (h0 | (h1 << 5) | (h2 << 10)) * 0x10001u | kGuard;
-    }
-    const uint32_t words[4] = {w4.x, w4.y, w4.z, w4.w};
-    unsigned hit = 0;
+__device__ __forceinline__ uint4 load_codes(const GridView& g, int p, int lane) {
+  return __ldg(reinterpret_cast<const uint4*>(g.codes) + (p >> 3) + lane);
+}
+
+// Hits among the 256 codes at pw (lane: 8 of them in w), of those in [p0, p1).
+__device__ __forceinline__ unsigned code_hits(const uint4& w, uint32_t lo, uint32_t hi, int q0,
+                                              int p0, int p1) {
+  const uint32_t words[4] = {w.x, w.y, w.z, w.w};
+  unsigned hit = 0;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      // a guard bit survives both subtractions where lo <= field <= hi
-      const uint32_t m = (((words[j] | kGuard) - lo) & (hi - words[j]) & kGuard) ^ kGuard;
-      hit |= ((m & 0xffffu) == 0u ? 1u : 0u) << (2 * j);
-      hit |= ((m >> 16) == 0u ? 1u : 0u) << (2 * j + 1);
-    }
-    const int q0 = pw + 8 * lane;
-    if (q0 < p0) hit &= p0 - q0 < 8 ? 0xffu << (p0 - q0) : 0u;
-    if (q0 + 8 > p1) hit &= p1 > q0 ? 0xffu >> (8 - (p1 - q0)) : 0u;
-    const int incl = warp_inclusive(__popc(hit), lane);
-    const int tot = __shfl_sync(kAll, incl, 31);
-    if (tot == 0) continue;
-    if (nbuf + tot > kHits) {
-      if (!take_hits<kIdx>(g, b, W, r, lane, qx, qy, qz, nbuf, k)) return false;
-      nbuf = 0;
-      if (tot > kHits) {
-        if (!take_range<kIdx>(g, b, W, r, lane, qx, qy, qz, max(pw, p0), min(pw + 256, p1), k))
-          return false;
-        continue;
-      }
-    }
-    int pos = nbuf + incl - __popc(hit);
-    while (hit) {
-      W.hits[pos++] = q0 + __ffs(hit) - 1;
-      hit &= hit - 1;
-    }
-    nbuf += tot;
-    if (nbuf >= 32) {
-      if (!take_hits<kIdx>(g, b, W, r, lane, qx, qy, qz, nbuf, k)) return false;
-      nbuf = 0;
-    }
+  for (int j = 0; j < 4; ++j) {
+    // a guard bit survives both subtractions where lo <= field <= hi
+    const uint32_t m = (((words[j] | kGuard) - lo) & (hi - words[j]) & kGuard) ^ kGuard;
+    hit |= ((m & 0xffffu) == 0u ? 1u : 0u) << (2 * j);
+    hit |= ((m >> 16) == 0u ? 1u : 0u) << (2 * j + 1);
   }
-  return take_hits<kIdx>(g, b, W, r, lane, qx, qy, qz, nbuf, k);
+  if (q0 < p0) hit &= p0 - q0 < 8 ? 0xffu << (p0 - q0) : 0u;
+  if (q0 + 8 > p1) hit &= p1 > q0 ? 0xffu >> (8 - (p1 - q0)) : 0u;
+  return hit;
 }
 
 // Cell `it` of the spiral around (cx, cy, cz).
@@ -356,13 +267,12 @@ __device__ __forceinline__ SpiralCell spiral_cell(const GridView& g,
 
 // Builds ray r's list for the points at z in [za, zb] of the ray o + z l, all
 // located in cell (cx, cy, cz), subcell `sub`. All arguments are warp-uniform.
-// Returns false when the range has to be narrowed.
+// Returns the candidates looked at, or -1 when the range has to be narrowed.
 template <bool kIdx>
-__device__ __forceinline__ bool build_list(const GridView& g, const char4* __restrict__ spiral,
+__device__ __forceinline__ int build_list(const GridView& g, const char4* __restrict__ spiral,
                                            WarpLists& W, int r, int lane, float ox, float oy,
                                            float oz, float lx, float ly, float lz, float len_l,
-                                           int cx, int cy, int cz, int sub, float za, float zb,
-                                           int& tested) {
+                                           int cx, int cy, int cz, int sub, float za, float zb) {
   const char4* order = spiral + sub * 125;
   const float zc = za + 0.5f * (zb - za);
   const float qx = ox + zc * lx, qy = oy + zc * ly, qz = oz + zc * lz;
@@ -370,14 +280,14 @@ __device__ __forceinline__ bool build_list(const GridView& g, const char4* __res
   const float del = ((fabsf(ox) + fabsf(oy)) + (fabsf(oz) + fabsf(zb) * len_l)) * 9.5367432e-7f;
   const float bb = 0.5f * (zb - za) * len_l * 1.00001f + del;
   const float crad = g.cell_radius;
-  if (!(bb < 1e15f) || !(crad < 1e15f)) return false;
+  if (!(bb < 1e15f) || !(crad < 1e15f)) return -1;
   BuildState b;
   b.s8 = __int_as_float(0x7f800000);
   b.R2 = b.R = b.T2 = b.s8;
   b.tb = 2.0f * bb;
   b.n = 0;
   b.seeded = false;
-  tested = 0;
+  int tested = 0;
   SpiralCell first;
   int kend = 125;  // cells from here on are not visited
   __syncwarp();
@@ -390,35 +300,99 @@ __device__ __forceinline__ bool build_list(const GridView& g, const char4* __res
     const float gy = fmaxf(fabsf(s.ccy - qy) - g.half1 - g.margin, 0.0f);
     const float gz = fmaxf(fabsf(s.ccz - qz) - g.half2 - g.margin, 0.0f);
     const float box2 = ((gx * gx + gy * gy) + gz * gz) * 0.99999f;
-    int cur = 0;
-    unsigned brk;
+    int cur = 0;          // first cell not taken yet
+    int q = 0, qe = 0;    // candidates to load next
+    int cp = 0, ce = 0;   // candidates to read through their codes next
+    int cell = 0;         // their cell's lane
+    int hb = 0, he = 0;   // buffered hits
+    uint4 nx;             // the codes at cp & ~7
+    unsigned brk = 0;
+    // one batch of up to 32 candidates in walk order per turn
 #pragma unroll 1
     for (;;) {
-      // cells from the first at which every point surely breaks are not visited
-      brk = __ballot_sync(
-          kAll, s.valid && lane >= cur && s.D - bb > (b.R + bb + crad) * 1.00001f);
-      const int kb = brk ? __ffs(brk) - 1 : 32;
-      const bool el = s.nc > 0 && lane >= cur && lane < kb && box2 <= b.T2;
-      const unsigned em = __ballot_sync(kAll, el);
-      if (!em) break;
-      const int incl = warp_inclusive(el ? min(s.nc, 33) : 0, lane);
-      const bool in = el && incl <= 32;
-      const unsigned bm = __ballot_sync(kAll, in);
-      const int f = __ffs(em) - 1;
-      if (!((bm >> f) & 1u)) {
-        // a cell with more than 32 candidates
-        const int p0 = __shfl_sync(kAll, s.b0, f), p1 = p0 + __shfl_sync(kAll, s.nc, f);
-        tested += p1 - p0;
-        const bool coded = p1 - p0 > kCodedMin;
-        const int pd = coded ? p0 + kDirect : p1;
-        if (!take_range<kIdx>(g, b, W, r, lane, qx, qy, qz, p0, pd, it0 + f)) return false;
-        if (coded && !take_coded<kIdx>(g, b, W, r, lane, qx, qy, qz,
-                                       __shfl_sync(kAll, s.ccx, f) - g.half0,
-                                       __shfl_sync(kAll, s.ccy, f) - g.half1,
-                                       __shfl_sync(kAll, s.ccz, f) - g.half2, pd, p1, it0 + f))
-          return false;
-        cur = f + 1;
+      bool valid;
+      int p, k;
+      if (q < qe) {
+        p = q + lane;
+        valid = p < qe;
+        if (!valid) p = q;
+        k = it0 + cell;
+        q += 32;
+      } else if (cp < ce || hb < he) {
+        const float e = b.T + g.margin;
+        uint32_t l0, h0, l1, h1, l2, h2;
+        const float mx = __shfl_sync(kAll, s.ccx, cell) - g.half0,
+                    my = __shfl_sync(kAll, s.ccy, cell) - g.half1,
+                    mz = __shfl_sync(kAll, s.ccz, cell) - g.half2;
+        // (none: no later candidate of the cell is within reach)
+        if (!(code_range(qx - e - mx, qx + e - mx, g.inv_w0, l0, h0) &
+              code_range(qy - e - my, qy + e - my, g.inv_w1, l1, h1) &
+              code_range(qz - e - mz, qz + e - mz, g.inv_w2, l2, h2))) {
+          cp = ce;
+          hb = he = 0;
+          continue;
+        }
+        const uint32_t lo = (l0 | (l1 << 5) | (l2 << 10)) * 0x10001u;
+        const uint32_t hi = (h0 | (h1 << 5) | (h2 << 10)) * 0x10001u | kGuard;
+#pragma unroll 1
+        while (cp < ce && he - hb < 32) {
+          const int pw = cp & ~7, q0 = pw + 8 * lane;
+          unsigned hit = code_hits(nx, lo, hi, q0, cp, ce);
+          const int incl = warp_inclusive(__popc(hit), lane);
+          const int tot = __shfl_sync(kAll, incl, 31);
+          if (tot > kHits - 32) {  // most of them: loaded without the codes
+            if (hb < he) break;    // (after the buffered ones)
+            q = cp;
+            qe = min(pw + 256, ce);
+          } else if (tot) {
+            if (he + tot > kHits) {  // the pending hits (fewer than 32) to the front
+              const int h = W.hits[min(hb + lane, kHits - 1)];
+              __syncwarp();
+              W.hits[lane] = h;
+              he -= hb;
+              hb = 0;
+              __syncwarp();
+            }
+            int pos = he + incl - __popc(hit);
+            while (hit) {
+              W.hits[pos++] = q0 + __ffs(hit) - 1;
+              hit &= hit - 1;
+            }
+            he += tot;
+          }
+          cp = min(pw + 256, ce);
+          if (cp < ce) nx = load_codes(g, cp, lane);
+          if (q < qe) break;
+        }
+        if (hb == he) continue;
+        __syncwarp();
+        k = it0 + cell;
+        valid = hb + lane < he;
+        p = W.hits[valid ? hb + lane : hb];
+        hb = min(hb + 32, he);
+        if (hb == he) hb = he = 0;
+        __syncwarp();
       } else {
+        // cells from the first at which every point surely breaks are not visited
+        brk = __ballot_sync(
+            kAll, s.valid && lane >= cur && s.D - bb > (b.R + bb + crad) * 1.00001f);
+        const int kb = brk ? __ffs(brk) - 1 : 32;
+        const bool el = s.nc > 0 && lane >= cur && lane < kb && box2 <= b.T2;
+        const unsigned em = __ballot_sync(kAll, el);
+        if (!em) break;
+        const int incl = warp_inclusive(el ? min(s.nc, 33) : 0, lane);
+        const bool in = el && incl <= 32;
+        const unsigned bm = __ballot_sync(kAll, in);
+        cell = __ffs(em) - 1;
+        if (!((bm >> cell) & 1u)) {  // a cell with more than 32 candidates
+          q = __shfl_sync(kAll, s.b0, cell);
+          ce = q + __shfl_sync(kAll, s.nc, cell);
+          tested += ce - q;
+          qe = cp = ce - q > kCodedMin ? q + kDirect : ce;
+          if (cp < ce) nx = load_codes(g, cp, lane);
+          cur = cell + 1;
+          continue;
+        }
         // the next whole cells that together have at most 32 candidates
         const int lastl = 31 - __clz(bm);
         const int tot = __shfl_sync(kAll, incl, lastl);
@@ -427,17 +401,20 @@ __device__ __forceinline__ bool build_list(const GridView& g, const char4* __res
         const unsigned starts = __reduce_or_sync(kAll, in ? 1u << excl : 0u);
         __syncwarp();
         const int src = W.owner[__popc(starts & (0xffffffffu >> (31 - lane))) - 1];
-        const int p = __shfl_sync(kAll, s.b0 - excl, src) + lane;
-        const bool valid = lane < tot;
-        const float4 P = __ldg(&g.parts[valid ? p : 0]);
-        const float fx = P.x - qx, fy = P.y - qy, fz = P.z - qz;
-        const float d2 = (fx * fx + fy * fy) + fz * fz;
+        p = __shfl_sync(kAll, s.b0 - excl, src) + lane;
+        valid = lane < tot;
+        if (!valid) p = 0;
+        k = it0 + src;
         tested += tot;
-        build_take<kIdx>(g, b, W, r, lane, valid, P, d2, p, it0 + src);
-        if (b.n > kCapAll) return false;
         cur = lastl + 1;
         __syncwarp();
       }
+      const float4 P = __ldg(&g.parts[p]);
+      const float fx = P.x - qx, fy = P.y - qy, fz = P.z - qz;
+      const float d2 = (fx * fx + fy * fy) + fz * fz;
+      if (!__any_sync(kAll, valid && d2 < b.T2)) continue;
+      build_take<kIdx>(g, b, W, r, lane, valid, P, d2, p, k);
+      if (b.n > kCapAll) return -1;
     }
     if (brk) {
       kend = it0 + __ffs(brk) - 1;
@@ -470,7 +447,7 @@ __device__ __forceinline__ bool build_list(const GridView& g, const char4* __res
     cells_run += __popc(ingm);
     cands_run += (uint32_t)__shfl_sync(kAll, incl, 31);
   }
-  if (nu > kUnc) return false;
+  if (nu > kUnc) return -1;
   __syncwarp();
   // candidates before the first of them, and up to each next one
   const int ku = W.owner[0];
@@ -497,9 +474,10 @@ __device__ __forceinline__ bool build_list(const GridView& g, const char4* __res
     m.zb = zb;
     m.n = n;
     m.nu = nu;
+    m.all = b.n;
   }
   __syncwarp();
-  return true;
+  return tested;
 }
 
 // A lane's slots after its point's walk: distances and values (indices).
@@ -507,74 +485,106 @@ struct PointSlots {
   float d[8], v[8];
 };
 
+__device__ __forceinline__ float max8(const float d[8]) {
+  return fmaxf(fmaxf(fmaxf(d[0], d[1]), fmaxf(d[2], d[3])),
+               fmaxf(fmaxf(d[4], d[5]), fmaxf(d[6], d[7])));
+}
+
 // Replays the walk of the point (x, y, z) over ray r's list.
+//
+// The walk compares rounded distances and replaces the first maximal slot.
+// Squared distances order the same way unless two of them lie within a few
+// ulp of each other (their roots may then be equal) or are equal, which
+// matters only for the slot maximum and the candidate that replaces it: the
+// new maximum is then within 2^-21 of the old one. The replay runs on squared
+// distances, with 8 square roots at the end; where that happened (or slots may
+// stay empty) it runs again on the distances themselves.
 template <bool kIdx>
 __device__ __forceinline__ void replay_point(const GridView& g, const WarpLists& W, int r,
                                              float x, float y, float z, PointSlots& o,
                                              WalkStats& st) {
-  const float4* __restrict__ E = W.ent[r];
-  const int n = W.meta[r].n;
-  int ix[8];
-  // the first 8 candidates fill the slots
-  float R = 0.0f;
+  const RayMeta& m = W.meta[r];
+  const int n = m.n, nu = m.nu;
+  bool exact = n < 8;
+  int ix[8], u;
+  for (;;) {
+    // the first 8 candidates fill the slots
 #pragma unroll
-  for (int t = 0; t < 8; ++t) {
-    o.d[t] = FLT_MAX;
-    ix[t] = t;
-    if (t < n) {
-      const float4 P = E[t];
+    for (int t = 0; t < 8; ++t) {
+      const float4 P = W.ent[r][t];
       const float fx = P.x - x, fy = P.y - y, fz = P.z - z;
-      o.d[t] = sqrtf((fx * fx + fy * fy) + fz * fz);
+      o.d[t] = (fx * fx + fy * fy) + fz * fz;
+      ix[t] = t;
     }
-    R = fmaxf(R, o.d[t]);
-  }
-  float R2 = __fmul_ru(R, R);
-  auto take = [&](const float4& P, int t) {
-    const float fx = P.x - x, fy = P.y - y, fz = P.z - z;
-    const float d2 = (fx * fx + fy * fy) + fz * fz;
-    if (d2 <= R2) {
-      const float dist = sqrtf(d2);
-      if (dist < R) {  // replace the first maximal slot
-        bool done = false;
-        float m = 0.0f;
+    if (exact) {
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          const bool hit = !done && o.d[q] == R;
-          done = done || hit;
-          o.d[q] = hit ? dist : o.d[q];
-          ix[q] = hit ? t : ix[q];
-          m = fmaxf(m, o.d[q]);
-        }
-        R = m;
-        R2 = __fmul_ru(R, R);
-      }
+      for (int t = 0; t < 8; ++t) o.d[t] = t < n ? sqrtf(o.d[t]) : FLT_MAX;
     }
-  };
-  const int n0 = min(n, kCap);
-  float4 P = E[8 < n ? 8 : 0];
+    float M = max8(o.d);                       // the slot maximum
+    float T = exact ? __fmul_ru(M, M) : M;     // squared distances above it cannot enter
+    bool close = false;
+    int t = min(8, n), end = n;
+    u = 0;
+    for (;;) {
 #pragma unroll 1
-  for (int t = 8; t < n0; ++t) {
-    const float4 C = P;
-    P = E[t + 1];
-    take(C, t);
-  }
-  for (int t = kCap; t < n; ++t) take(list_entry(W, r, t), t);
-  // the break, cell by cell (the last one breaks every point)
-  const int nu = W.meta[r].nu;
-  int u = 0, t = n;
-  for (; u < nu - 1; ++u) {
-    const float4 c = W.unc[r][u];
-    const float ex = c.x - x, ey = c.y - y, ez = c.z - z;
-    const float rb = R + g.cell_radius;
-    if ((ex * ex + ey * ey) + ez * ez > rb * rb) break;
-    const int end = (int)((__float_as_uint(c.w) >> 8) & 0xffu);
-    for (; t < end; ++t) take(list_entry(W, r, t), t);
+      for (; t < end; ++t) {
+        const float4 P = list_entry(W, r, t);
+        const float fx = P.x - x, fy = P.y - y, fz = P.z - z;
+        float d = (fx * fx + fy * fy) + fz * fz;
+        if (d <= T) {
+          if (exact) d = sqrtf(d);
+          if (d < M) {
+            bool open = true;
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+              const bool eq = o.d[q] == M;
+              const bool hit = open && eq;
+              open = open && !eq;
+              o.d[q] = hit ? d : o.d[q];
+              ix[q] = hit ? t : ix[q];
+            }
+            const float top = max8(o.d);
+            close = close || top >= M * 0.99999952f;
+            M = top;
+            T = exact ? __fmul_ru(M, M) : M;
+          }
+        }
+      }
+      // the break, cell by cell (the last one breaks every point)
+      const float rb = (exact ? M : sqrtf(M)) + g.cell_radius;
+      const float rr = rb * rb;
+      bool more = false;
+#pragma unroll 1
+      for (; u < nu - 1; ++u) {
+        const float4 c = W.unc[r][u];
+        const float ex = c.x - x, ey = c.y - y, ez = c.z - z;
+        if ((ex * ex + ey * ey) + ez * ez > rr) break;
+        end = (int)((__float_as_uint(c.w) >> 8) & 0xffu);
+        if (t < end) {
+          more = true;
+          ++u;
+          break;
+        }
+      }
+      if (!more) break;
+    }
+    if (exact || !close) break;
+    exact = true;
   }
   st.cells += __float_as_uint(W.unc[r][u].w) & 0xffu;
   st.cands += W.unp[r][u];
+  if (m.all <= kCap && n >= 8) {
 #pragma unroll
-  for (int q = 0; q < 8; ++q)
-    o.v[q] = o.d[q] < FLT_MAX ? list_entry(W, r, ix[q]).w : (kIdx ? __int_as_float(-1) : 0.0f);
+    for (int q = 0; q < 8; ++q) o.v[q] = W.ent[r][ix[q]].w;
+  } else {
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      o.v[q] = o.d[q] < FLT_MAX ? list_entry(W, r, ix[q]).w : (kIdx ? __int_as_float(-1) : 0.0f);
+  }
+  if (!exact) {
+#pragma unroll
+    for (int q = 0; q < 8; ++q) o.d[q] = sqrtf(o.d[q]);
+  }
 }
 
 // nn8 slots of the lanes' points: lane 4r + j holds point j of ray r at
@@ -589,26 +599,33 @@ __device__ __forceinline__ void eval_points(const GridView& g, const char4* __re
   const int r = lane >> 2;
   const unsigned mine = 0xfu << (lane & 28);
   bool todo = active;
-  bool listed = false;
   for (;;) {
+    bool listed = false;
     if (todo) {
       const RayMeta& m = W.meta[r];
       listed = zq >= m.za && zq <= m.zb;
-    } else {
-      listed = false;
     }
-    const unsigned lm = __ballot_sync(kAll, listed);
-    unsigned need = __ballot_sync(kAll, todo && !(lm & mine));
-    if (need) {
+    const unsigned lm = __ballot_sync(kAll, listed) & mine;
+    const unsigned todom = __ballot_sync(kAll, todo), rm = todom & mine;
+    // rays with a point that their list does not hold for: all of their
+    // points get a new list if they share their cell and subcell, otherwise
+    // the listed points go first
+    const bool part = todo && lm != rm;
+    if (__any_sync(kAll, part)) {
       int cx = 0, cy = 0, cz = 0, sub = 0;
-      if ((need >> lane) & 1u) {
+      if (part) {
         int sx, sy, sz;
         locate_axis(x, g.min0, g.cs0, g.half0, cx, sx);
         locate_axis(y, g.min1, g.cs1, g.half1, cy, sy);
         locate_axis(z, g.min2, g.cs2, g.half2, cz, sz);
         sub = sx + 2 * sy + 4 * sz;
       }
-      const unsigned todom = __ballot_sync(kAll, todo);
+      const int rl = rm ? __ffs(rm) - 1 : lane;
+      const int fx = __shfl_sync(kAll, cx, rl), fy = __shfl_sync(kAll, cy, rl),
+                fz = __shfl_sync(kAll, cz, rl), fs = __shfl_sync(kAll, sub, rl);
+      const bool same = part && cx == fx && cy == fy && cz == fz && sub == fs;
+      const unsigned sm = __ballot_sync(kAll, same) & mine;
+      unsigned need = __ballot_sync(kAll, part && (lm == 0u || sm == rm));
 #pragma unroll 1
       while (need) {
         const int lead = __ffs(need) - 1, lr = lead >> 2;
@@ -651,7 +668,7 @@ __device__ __forceinline__ void eval_points(const GridView& g, const char4* __re
                         g.half2, g.margin);
           const float reach = fminf(zlo + ext, fminf(ex, fminf(ey, ez)));
           float a = zlo, b = reach > zhi ? reach : zhi;
-          int tested = 0;
+          int tested = -1;
 #pragma unroll 1
           for (int attempt = 0; attempt < 3; ++attempt) {
             if (attempt == 1) {
@@ -662,14 +679,15 @@ __device__ __forceinline__ void eval_points(const GridView& g, const char4* __re
               if (!(zhi > zlo)) break;
               a = b = zl;
             }
-            ok = build_list<kIdx>(g, spiral, W, lr, lane, rox, roy, roz, rlx, rly, rlz,
-                                        len_l, bx, by, bz, bs, a, b, tested);
-            if (ok) break;
+            tested = build_list<kIdx>(g, spiral, W, lr, lane, rox, roy, roz, rlx, rly, rlz, len_l,
+                                      bx, by, bz, bs, a, b);
+            if (tested >= 0) break;
             ext *= 0.6f;
           }
           // longer lists pay where the search behind them is long
+          ok = tested >= 0;
           if (ok) {
-            const int n = W.meta[lr].n, want = tested > 256 ? kCapAll - 55 : 42;
+            const int n = W.meta[lr].n, want = tested > 256 ? 62 : 34;
             const int nu = W.meta[lr].nu;
             if (n > want || nu > kUnc - 4) ext *= 0.85f;
             else if (n < want - 8 && nu < kUnc - 8) ext *= 1.2f;
