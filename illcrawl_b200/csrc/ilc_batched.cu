@@ -104,9 +104,12 @@ __device__ __forceinline__ void ray_span(const JobDev& j, int ix, int iy, bool& 
 // One channel's FP64 step candidate: returns I + delta4 (as the accepted
 // value) and sets x to the channel's error ratio
 // max(atol, |I/z' rtol|) h / (2 |delta5 - delta4|), or 16 if delta4 == delta5.
+// rz = 1 / z', correctly rounded: I / z' is q + (I - q z') rz with q = I rz, each
+// one rounding, which is the correctly rounded quotient (Markstein's theorem;
+// I is a float, so nothing leaves the double range).
 __device__ __forceinline__ float channel_step(float Ic, float k1c, float e0, float e1, float e2,
-                                              float e3, double hd, float znew, double atol,
-                                              double rtol, double& x) {
+                                              float e3, double hd, double zd, double rz,
+                                              double atol, double rtol, double& x) {
   double d4 = 25.0 / 216.0 * (double)k1c + 1408.0 / 2565.0 * (double)e0 +
               2197.0 / 4101.0 * (double)e1 - 1.0 / 5.0 * (double)e2;
   double d5 = 16.0 / 135.0 * (double)k1c + 6656.0 / 12825.0 * (double)e0 +
@@ -116,7 +119,9 @@ __device__ __forceinline__ float channel_step(float Ic, float k1c, float e0, flo
   x = 16.0;
   if (d4 != d5) {
     const double err = fabs(d5 - d4);
-    const double srt = fabs((double)Ic / (double)znew * rtol);
+    const double q = (double)Ic * rz;
+    const double quo = fabs(q) <= DBL_MAX ? fma(fma(-q, zd, (double)Ic), rz, q) : q;
+    const double srt = fabs(quo * rtol);
     const double ot = fmax(atol, srt);
     x = ot * hd / (2.0 * err);
   }
@@ -278,13 +283,16 @@ batched_kernel(const __grid_constant__ BatchK a, const __grid_constant__ GridVie
         float* Is = wstate + (size_t)tr * 4 * a.V;
         float* Ks = Is + a.V;
         const double hd = (double)hr;
-        const float znew = zr + hr;
+        const double zd = (double)(zr + hr), rz = 1.0 / zd;
         double xl = __longlong_as_double(0x7ff0000000000000ll);  // +inf
         bool x0nan = false;
-        // candidate values (I + delta4, k5) go to the ray's scratch half
-        // and are committed once the warp knows the step is accepted
+        // candidate values (I + delta4, k5): a lane's last group stays in
+        // registers, earlier ones (V > 128) go to the ray's scratch half; they
+        // are committed once the warp knows the step is accepted
         float* Es = Ks + a.V;
         float* E2s = Es + a.V;
+        int held = -1;
+        float4 hi4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f), hk4 = hi4;
         if ((a.V & 3) == 0) {
           // rows of V = 4G floats: lane handles float4 groups lane, lane+32, ...
           // (channels 4g..4g+3), one 16-byte load per neighbour and group
@@ -292,6 +300,13 @@ batched_kernel(const __grid_constant__ BatchK a, const __grid_constant__ GridVie
           const float4* __restrict__ chan4 = reinterpret_cast<const float4*>(a.chan);
 #pragma unroll 1
           for (int gi = lane; gi < G; gi += 32) {
+            if (held >= 0) {
+              reinterpret_cast<float4*>(Es)[held] = hi4;
+              reinterpret_cast<float4*>(E2s)[held] = hk4;
+            }
+            held = gi;
+            const float4 i4 = reinterpret_cast<const float4*>(Is)[gi];
+            const float4 k4 = reinterpret_cast<const float4*>(Ks)[gi];
             float ev[4][4];
 #pragma unroll
             for (int p = 0; p < 4; ++p) {
@@ -312,16 +327,18 @@ batched_kernel(const __grid_constant__ BatchK a, const __grid_constant__ GridVie
               for (int k = 0; k < 4; ++k)
                 ev[p][k] = (wsum != 0.0f && dot[k] != 0.0f) ? dot[k] / wsum : 0.0f;
             }
+            const float ic[4] = {i4.x, i4.y, i4.z, i4.w}, kc[4] = {k4.x, k4.y, k4.z, k4.w};
+            float en[4];
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-              const int c = 4 * gi + k;
               double x;
-              Es[c] = channel_step(Is[c], Ks[c], ev[0][k], ev[1][k], ev[2][k], ev[3][k], hd, znew,
-                                   a.atol, a.rtol, x);
-              E2s[c] = ev[2][k];
-              if (c == 0 && isnan(x)) x0nan = true;
+              en[k] = channel_step(ic[k], kc[k], ev[0][k], ev[1][k], ev[2][k], ev[3][k], hd, zd,
+                                   rz, a.atol, a.rtol, x);
+              if (gi == 0 && k == 0 && isnan(x)) x0nan = true;
               xl = fmin(xl, x);
             }
+            hi4 = make_float4(en[0], en[1], en[2], en[3]);
+            hk4 = make_float4(ev[2][0], ev[2][1], ev[2][2], ev[2][3]);
           }
         } else {
 #pragma unroll 1
@@ -340,7 +357,7 @@ batched_kernel(const __grid_constant__ BatchK a, const __grid_constant__ GridVie
               ev[p] = (wsum != 0.0f && dot != 0.0f) ? dot / wsum : 0.0f;
             }
             double x;
-            Es[c] = channel_step(Is[c], Ks[c], ev[0], ev[1], ev[2], ev[3], hd, znew, a.atol,
+            Es[c] = channel_step(Is[c], Ks[c], ev[0], ev[1], ev[2], ev[3], hd, zd, rz, a.atol,
                                  a.rtol, x);
             E2s[c] = ev[2];
             if (c == 0 && isnan(x)) x0nan = true;
@@ -360,10 +377,20 @@ batched_kernel(const __grid_constant__ BatchK a, const __grid_constant__ GridVie
         sc = nh / hd;
         const bool accept = !(sc < 0.95);
         if (accept) {
+          if (held >= 0) {
+            reinterpret_cast<float4*>(Is)[held] = hi4;
+            reinterpret_cast<float4*>(Ks)[held] = hk4;
 #pragma unroll 1
-          for (int c = lane; c < a.V; c += 32) {
-            Is[c] = Es[c];
-            Ks[c] = E2s[c];
+            for (int gi = lane; gi < held; gi += 32) {
+              reinterpret_cast<float4*>(Is)[gi] = reinterpret_cast<const float4*>(Es)[gi];
+              reinterpret_cast<float4*>(Ks)[gi] = reinterpret_cast<const float4*>(E2s)[gi];
+            }
+          } else if ((a.V & 3) != 0) {
+#pragma unroll 1
+            for (int c = lane; c < a.V; c += 32) {
+              Is[c] = Es[c];
+              Ks[c] = E2s[c];
+            }
           }
         }
         if (r == tr) {
