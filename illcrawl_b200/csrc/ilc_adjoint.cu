@@ -33,7 +33,7 @@ __device__ void band_flux_tangent(const float* t, const GauntView& G, float Emin
   float I = 0.0f, z = Emin, h = (Emax - Emin) * reltol;
   double dI = 0, dz = 0, dh = 0, dk1, dkE;
   const float end = Emax;
-  float k1 = brems(t, G, z, 1.0f, T, xe, rho, dL);
+  float k1 = brems(t, G, z, 1.0f, T, xe, rho, dL, G.w);
   brems_tangent(t, GD, z, T, xe, rho, dL, kWhich, &dk1, &dkE, (double)k1);
   float p[4];
   double dp[4] = {0, 0, 0, 0};
@@ -45,7 +45,7 @@ __device__ void band_flux_tangent(const float* t, const GauntView& G, float Emin
     double de[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      e[j] = brems(t, G, p[j], 1.0f, T, xe, rho, dL);
+      e[j] = brems(t, G, p[j], 1.0f, T, xe, rho, dL, G.w);
       double pl, pe;
       brems_tangent(t, GD, p[j], T, xe, rho, dL, kWhich, &pl, &pe, (double)e[j]);
       de[j] = pl + pe * dp[j];

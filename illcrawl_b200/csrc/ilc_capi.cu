@@ -11,6 +11,7 @@
 #include <vector>
 
 #include "ilc_internal.h"
+#include "ilc_quantity.cuh"
 #include "ilc_random.cuh"
 
 struct ilc_ctx {
@@ -484,7 +485,7 @@ void ilc_destroy(ilc_ctx* h) {
   cudaSetDevice(c.device);
   if (c.stream) cudaStreamSynchronize(c.stream);
   for (DevBuf* b : {&c.tile_queue, &c.list_over, &c.parts, &c.cells, &c.s2u, &c.keys_a, &c.keys_b, &c.vals_a, &c.vals_b,
-                    &c.hist, &c.tmp_in, &c.gaunt, &c.list_d, &c.list_v, &c.list_id, &c.in_a,
+                    &c.hist, &c.tmp_in, &c.gaunt, &c.gaunt_pad, &c.list_d, &c.list_v, &c.list_id, &c.in_a,
                     &c.in_b, &c.in_c, &c.out_a, &c.out_b, &c.out_c, &c.spiral, &c.flags,
                     &c.rec_h, &c.rec_n, &c.adj_dT, &c.adj_dR, &c.adj_grad, &c.adj_seed,
                     &c.adj_loss, &c.codes, &c.jobs, &c.chan_sorted, &c.chan_state, &c.queue,
@@ -637,8 +638,18 @@ ilc_status ilc_gaunt_load(ilc_ctx* h, const float* table, int32_t width, int32_t
       !(dy > 0.0f))
     return fail(c, ILC_ERR_INVALID_ARGUMENT, "invalid Gaunt table (at most 81 x 146 entries)");
   const size_t bytes = (size_t)width * height * 4;
+  const int pad = table_pad(width, height);
+  const size_t stride = (size_t)width + 2 * pad;
+  std::vector<float> padded((stride * ((size_t)height + 2 * pad) + 3) / 4 * 4, 0.0f);
+  for (int32_t j = 0; j < height; ++j)
+    std::memcpy(&padded[(size_t)(j + pad) * stride + pad], table + (size_t)j * width,
+                (size_t)width * 4);
   ILC_CUDA(c, c.gaunt.ensure(bytes), "gaunt alloc");
+  ILC_CUDA(c, c.gaunt_pad.ensure(padded.size() * 4), "gaunt alloc");
   ILC_CUDA(c, cudaMemcpyAsync(c.gaunt.p, table, bytes, cudaMemcpyHostToDevice, c.stream),
+           "gaunt H2D");
+  ILC_CUDA(c, cudaMemcpyAsync(c.gaunt_pad.p, padded.data(), padded.size() * 4,
+                              cudaMemcpyHostToDevice, c.stream),
            "gaunt H2D");
   ILC_CUDA(c, cudaStreamSynchronize(c.stream), "gaunt");
   c.gw = width; c.gh = height; c.gx0 = x0; c.gy0 = y0; c.gdx = dx; c.gdy = dy;

@@ -71,6 +71,7 @@ struct Context {
   // Gaunt table
   bool has_gaunt = false;
   DevBuf gaunt;
+  DevBuf gaunt_pad;  // the same with two rows and columns of zeros around it
   int32_t gw = 0, gh = 0;
   float gx0 = 0, gy0 = 0, gdx = 0, gdy = 0;
 
