@@ -484,7 +484,7 @@ void ilc_destroy(ilc_ctx* h) {
   Context& c = h->c;
   cudaSetDevice(c.device);
   if (c.stream) cudaStreamSynchronize(c.stream);
-  for (DevBuf* b : {&c.tile_queue, &c.list_over, &c.parts, &c.cells, &c.s2u, &c.keys_a, &c.keys_b, &c.vals_a, &c.vals_b,
+  for (DevBuf* b : {&c.tile_queue, &c.list_over, &c.query_sort, &c.parts, &c.cells, &c.s2u, &c.keys_a, &c.keys_b, &c.vals_a, &c.vals_b,
                     &c.hist, &c.tmp_in, &c.gaunt, &c.gaunt_pad, &c.list_d, &c.list_v, &c.list_id, &c.in_a,
                     &c.in_b, &c.in_c, &c.out_a, &c.out_b, &c.out_c, &c.spiral, &c.flags,
                     &c.rec_h, &c.rec_n, &c.adj_dT, &c.adj_dR, &c.adj_grad, &c.adj_seed,

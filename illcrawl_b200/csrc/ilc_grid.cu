@@ -389,6 +389,13 @@ cudaError_t exclusive_scan_u32(Context& c, uint32_t* a, uint64_t m) {
   return cudaGetLastError();
 }
 
+uint64_t scan_scratch_words(uint64_t m) { return scan_chunks(m); }
+
+cudaError_t exclusive_scan_long(Context& c, uint32_t* a, uint64_t m, uint32_t* scratch) {
+  c.launches += scan_u32(a, m, scratch, c.stream);
+  return cudaGetLastError();
+}
+
 cudaError_t grid_build_device(Context& c, const float4* in, uint64_t n) {
   cudaError_t e;
   const GridParams& g = c.gp;

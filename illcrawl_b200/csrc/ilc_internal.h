@@ -83,6 +83,7 @@ struct Context {
 
   // nn8 running lists for multi-block merging (volumetric_reconstruction_backend_nn8.cpp:57-66)
   DevBuf list_d, list_v, list_id;
+  DevBuf query_sort;  // counting sort of the queries by bin
   uint64_t list_n = 0;
 
   // generic per-call staging
@@ -136,6 +137,10 @@ cudaError_t grid_bbox(Context& c, const float4* in, uint64_t n, float* mn3, floa
 cudaError_t grid_build_device(Context& c, const float4* in, uint64_t n);
 // In-place exclusive prefix sum of m uint32 (one block; for per-block counts).
 cudaError_t exclusive_scan_u32(Context& c, uint32_t* a, uint64_t m);
+// The same over all SMs for long arrays (a 16-byte aligned); `scratch` holds
+// scan_scratch_words(m) words.
+uint64_t scan_scratch_words(uint64_t m);
+cudaError_t exclusive_scan_long(Context& c, uint32_t* a, uint64_t m, uint32_t* scratch);
 
 // Cell ingestion (ilc_ingest.cu): periodic correction and volume cutout of
 // n cells, compacted in input order into (x, y, z, q) float4 and the original

@@ -122,10 +122,12 @@ ilc_status ilc_set_render_engine(ilc_ctx* ctx, int32_t engine);
 
 /* Kernel of ilc_nn8_query (and of the consumers that query through it):
  * ILC_QUERY_THREAD (default) walks each query in one thread, as the
- * reference's kernel does; ILC_QUERY_WARP walks each query with a whole warp
- * (the cells of the spiral and the candidates tested 32 at a time, hits
- * collected by ballot and inserted in candidate order). Both give the same
- * results bit for bit. No reference counterpart. */
+ * reference's kernel does, where there are enough queries to fill the device
+ * that way, and leaves to the warp kernel the queries that meet a dense cell;
+ * ILC_QUERY_WARP walks every query with a whole warp (the cells of the spiral
+ * and the candidates tested 32 at a time, hits collected by ballot and inserted
+ * in candidate order). Both give the same results bit for bit. No reference
+ * counterpart. */
 enum { ILC_QUERY_THREAD = 0, ILC_QUERY_WARP = 1 };
 ilc_status ilc_set_query_engine(ilc_ctx* ctx, int32_t engine);
 
