@@ -252,22 +252,29 @@ nn8_query_kernel(const __grid_constant__ GridView g, const char4* __restrict__ s
 // as in the one-thread walk, and the result is the same bit for bit. The
 // maximum slot is found with __reduce_max_sync over the distances' bit
 // patterns (non-negative floats order as unsigned integers) and the first slot
-// holding it with a ballot. 1,000 queries of 20,000 particles: 322 -> 34 us;
-// 65,537 of 1,000,003: 1,833 -> 181 us (one lane per query before).
+// holding it with a ballot. 1,000 queries of 20,000 particles: 322 -> 37 us;
+// 65,537 of 1,000,003: 1,833 -> 168 us (one lane per query before; 184 us with
+// a square root and a copy of the value per insertion).
 // ---------------------------------------------------------------------------
+// This lane's slot (lanes 0-7): squared distance, or (exact) distance, and
+// candidate. M: the slot maximum, mi its first slot, T: squared distances above
+// it cannot enter, rr: the early-break threshold.
 struct WarpSlots {
-  float d, v;   // this lane's slot (lanes 0-7)
+  float d;
   int32_t id;
-  float R, R2up, rr;
+  float M, T, rr;
   int mi;
 };
 
-__device__ __forceinline__ void warp_rescan(WarpSlots& s, int lane, float crad) {
+__device__ __forceinline__ void warp_rescan(WarpSlots& s, int lane, bool exact) {
   const unsigned bits = __reduce_max_sync(kAll, lane < 8 ? __float_as_uint(s.d) : 0u);
-  s.R = __uint_as_float(bits);
+  s.M = __uint_as_float(bits);
   s.mi = __ffs(__ballot_sync(kAll, lane < 8 && __float_as_uint(s.d) == bits)) - 1;
-  s.R2up = __fmul_ru(s.R, s.R);
-  const float b = s.R + crad;
+  s.T = exact ? __fmul_ru(s.M, s.M) : s.M;
+}
+
+__device__ __forceinline__ void warp_break_radius(WarpSlots& s, float crad, bool exact) {
+  const float b = (exact ? s.M : fminf(sqrtf(s.M), FLT_MAX)) + crad;
   s.rr = b * b;
 }
 
@@ -276,15 +283,20 @@ struct QueryWarpMem {
   int hits[kHits];
 };
 
-__device__ __forceinline__ void nn8_walk_warp(const GridView& g, const char4* __restrict__ spiral,
+// exact: on rounded distances, as the reference; otherwise on squared ones (as
+// in a list replay), returning false where two are too close for that.
+__device__ __forceinline__ bool nn8_walk_warp(const GridView& g, const char4* __restrict__ spiral,
                                               QueryWarpMem& W, float qx, float qy, float qz,
-                                              WarpSlots& s, int lane, WalkStats& st) {
+                                              WarpSlots& s, int lane, bool exact,
+                                              WalkStats& st) {
   int cx, cy, cz, sx, sy, sz;
   locate_axis(qx, g.min0, g.cs0, g.half0, cx, sx);
   locate_axis(qy, g.min1, g.cs1, g.half1, cy, sy);
   locate_axis(qz, g.min2, g.cs2, g.half2, cz, sz);
   const char4* order = spiral + (sx + 2 * sy + 4 * sz) * 125;
-  const float crad = g.cell_radius;
+  const float crad = g.cell_radius, inf = __int_as_float(0x7f800000);
+  bool close = false;
+  warp_break_radius(s, crad, exact);
 #pragma unroll 1
   for (int it0 = 0; it0 < 125; it0 += 32) {
     // this lane's cell of the chunk
@@ -329,7 +341,7 @@ __device__ __forceinline__ void nn8_walk_warp(const GridView& g, const char4* __
         k = cell;
         q += 32;
       } else if (cp < ce || hb < he) {
-        const float e = s.R * 1.00001f + g.margin;
+        const float e = (exact ? s.M : sqrtf(s.M)) * 1.00001f + g.margin;
         uint32_t l0, h0, l1, h1, l2, h2;
         const float mx = __shfl_sync(kAll, ccx, cell) - g.half0,
                     my = __shfl_sync(kAll, ccy, cell) - g.half1,
@@ -385,7 +397,7 @@ __device__ __forceinline__ void nn8_walk_warp(const GridView& g, const char4* __
         // the cells up to the first due break with candidates within reach
         const unsigned bm = __ballot_sync(kAll, valid_cell && lane >= cur && cd > s.rr);
         const int kb = bm ? __ffs(bm) - 1 : 32;
-        const bool el = nc > 0 && lane >= cur && lane < kb && box2 <= s.R2up;
+        const bool el = nc > 0 && lane >= cur && lane < kb && box2 <= s.T;
         const unsigned em = __ballot_sync(kAll, el);
         if (!em) {
           if (bm) brk = kb;
@@ -420,13 +432,31 @@ __device__ __forceinline__ void nn8_walk_warp(const GridView& g, const char4* __
       const float fx = P.x - qx, fy = P.y - qy, fz = P.z - qz;
       const float d2 = (fx * fx + fy * fy) + fz * fz;
       int last = -1;
+      if (s.M == inf) {
+        // (not exact) empty slots: the first 8 candidates fill them, no break
+        // being possible before
+        const unsigned fm = __ballot_sync(kAll, valid && d2 < inf);
+        if ((fm & 0xffu) == 0xffu && __ballot_sync(kAll, lane < 8 && s.id != -1) == 0u) {
+          if (lane < 8) {
+            s.d = d2;
+            s.id = p;
+          }
+          warp_rescan(s, lane, exact);
+          cur = max(cur, __shfl_sync(kAll, k, 7) + 1);
+          last = 7;
+          warp_break_radius(s, crad, exact);
+        }
+      }
+      bool stale = false;  // rr is behind M
       for (;;) {
-        const unsigned hm = __ballot_sync(kAll, valid && lane > last && d2 <= s.R2up);
+        const unsigned hm = __ballot_sync(kAll, valid && lane > last && d2 <= s.T);
         if (!hm) break;
         const int i = __ffs(hm) - 1;
         last = i;
         const int ck = __shfl_sync(kAll, k, i);
         if (ck >= cur) {  // break tests of the cells up to this candidate's cell
+          if (stale) warp_break_radius(s, crad, exact);
+          stale = false;
           const unsigned due = __ballot_sync(kAll, valid_cell && lane >= cur && lane <= ck &&
                                                        cd > s.rr);
           if (due) {
@@ -435,18 +465,21 @@ __device__ __forceinline__ void nn8_walk_warp(const GridView& g, const char4* __
           }
           cur = ck + 1;
         }
-        const float dist = sqrtf(__shfl_sync(kAll, d2, i));
-        if (dist < s.R) {
-          const float vk = __shfl_sync(kAll, P.w, i);
+        float d = __shfl_sync(kAll, d2, i);
+        if (exact) d = sqrtf(d);
+        if (d < s.M) {
           const int pk = __shfl_sync(kAll, p, i);
           if (lane == s.mi) {
-            s.d = dist;
-            s.v = vk;
+            s.d = d;
             s.id = pk;
           }
-          warp_rescan(s, lane, crad);
+          const float before = s.M;
+          warp_rescan(s, lane, exact);
+          close = close || (before < inf && s.M >= before * 0.99999952f);
+          stale = true;
         }
       }
+      if (stale) warp_break_radius(s, crad, exact);
       if (brk >= 0) break;
       if (q >= qe && cp >= ce && hb >= he) {
         // the batch's cells are done: the break tests due at them
@@ -465,8 +498,9 @@ __device__ __forceinline__ void nn8_walk_warp(const GridView& g, const char4* __
     st.cells += __popc(__ballot_sync(kAll, ing && lane < seen));
     const int incl = warp_inclusive(lane < seen ? nc : 0, lane);
     st.cands += (uint32_t)__shfl_sync(kAll, incl, 31);
-    if (brk >= 0) return;
+    if (brk >= 0) break;
   }
+  return exact || !close;
 }
 
 // todo: the queries to take (nullptr: all n), n_todo of them (device counter).
@@ -492,20 +526,28 @@ nn8_query_warp_kernel(const __grid_constant__ GridView g, const char4* __restric
     const uint64_t i = todo ? todo[turn] : turn;
     const float4 q = pts[i];
     WarpSlots s;
-    s.d = FLT_MAX;
-    s.v = 0.0f;
-    s.id = -1;
-    if (merge && lane < 8) {
-      s.d = list_d[8 * i + lane];
-      s.v = list_v[8 * i + lane];
-      const int32_t o = list_id[8 * i + lane];
-      s.id = o >= 0 ? (int32_t)(0x80000000u | (uint32_t)o) : -1;
+    bool exact = merge != 0;
+    for (;;) {
+      s.d = exact ? FLT_MAX : __int_as_float(0x7f800000);
+      s.id = -1;
+      if (merge && lane < 8) {
+        s.d = list_d[8 * i + lane];
+        const int32_t o = list_id[8 * i + lane];
+        s.id = o >= 0 ? (int32_t)(0x80000000u | (uint32_t)o) : -1;
+      }
+      warp_rescan(s, lane, exact);
+      st.cells = st.cands = 0;
+      if (nn8_walk_warp(g, spiral, mem[threadIdx.x >> 5], q.x, q.y, q.z, s, lane, exact, st))
+        break;
+      exact = true;
     }
-    warp_rescan(s, lane, g.cell_radius);
-    st.cells = st.cands = 0;
-    nn8_walk_warp(g, spiral, mem[threadIdx.x >> 5], q.x, q.y, q.z, s, lane, st);
     cells += st.cells;
     cands += st.cands;
+    if (!exact) s.d = s.id < 0 ? FLT_MAX : sqrtf(s.d);
+    // a slot not replaced keeps its list entry
+    float v = 0.0f;
+    if (lane < 8 && s.id >= 0) v = __ldg(&g.parts[s.id].w);
+    else if (lane < 8 && merge) v = list_v[8 * i + lane];
     // finalize in slot order (volumetric_nn8_reconstruction.cl:212-270)
     const float w = weight3d(s.d);
     float ws = 0.0f, dot = 0.0f;
@@ -513,14 +555,14 @@ nn8_query_warp_kernel(const __grid_constant__ GridView g, const char4* __restric
     for (int t = 0; t < 8; ++t) ws = ws + __shfl_sync(kAll, w, t);
 #pragma unroll
     for (int t = 0; t < 8; ++t)
-      dot = __fmaf_rn(__shfl_sync(kAll, w, t), __shfl_sync(kAll, s.v, t), dot);
+      dot = __fmaf_rn(__shfl_sync(kAll, w, t), __shfl_sync(kAll, v, t), dot);
     if (lane == 0) out[i] = (ws != 0.0f && dot != 0.0f) ? dot / ws : 0.0f;
     if (lane < 8) {
       const int32_t id = s.id;
       const int32_t orig =
           id == -1 ? -1 : (id < 0 ? (int32_t)((uint32_t)id & 0x7fffffffu) : (int32_t)s2u[id]);
       list_d[8 * i + lane] = s.d;
-      list_v[8 * i + lane] = s.v;
+      list_v[8 * i + lane] = v;
       list_id[8 * i + lane] = orig;
       if (idx8) idx8[8 * i + lane] = orig;
       if (d8) d8[8 * i + lane] = s.d;
