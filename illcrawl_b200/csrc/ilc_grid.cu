@@ -3,8 +3,9 @@
 //
 // Pipeline: bounding box (exact float min/max) -> host grid parameters in
 // double, as the reference -> cell keys -> stable LSD radix sort of (key,
-// original index) -> gather of the float4 particles into cell order -> cell
-// [begin, end) ranges by adjacent difference over a zero-filled cell array.
+// original index) -> one pass that gathers the float4 particles into cell
+// order and writes the cell [begin, end) ranges (by adjacent difference over a
+// zero-filled cell array) and sub-box codes.
 // The stable sort gives the permutation boost::compute::sort_by_key gives, so
 // keys, permutation and cell ranges are bit-identical to the reference's.
 #include <algorithm>
@@ -57,13 +58,27 @@ __global__ void bbox_kernel(const float4* __restrict__ in, uint64_t n, unsigned*
     }
   }
   bad = __any_sync(0xffffffffu, bad);
+  // one set of atomics per block: those of every warp queued up on the seven
+  // words (42 us of 1,000,003 particles' box; now 6)
+  __shared__ unsigned part[32][7];
   if ((threadIdx.x & 31) == 0) {
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-      atomicMin(&acc[k], mn[k]);
-      atomicMax(&acc[3 + k], mx[k]);
+      part[threadIdx.x >> 5][k] = mn[k];
+      part[threadIdx.x >> 5][3 + k] = mx[k];
     }
-    if (bad) atomicOr(&acc[6], 1u);
+    part[threadIdx.x >> 5][6] = bad;
+  }
+  __syncthreads();
+  if (threadIdx.x < 7) {
+    unsigned v = part[0][threadIdx.x];
+    for (unsigned w = 1; w < blockDim.x / 32; ++w) {
+      const unsigned o = part[w][threadIdx.x];
+      v = threadIdx.x < 3 ? min(v, o) : max(v, o);
+    }
+    if (threadIdx.x < 3) atomicMin(&acc[threadIdx.x], v);
+    else if (threadIdx.x < 6) atomicMax(&acc[threadIdx.x], v);
+    else if (v) atomicOr(&acc[6], 1u);
   }
 }
 
@@ -95,26 +110,29 @@ __global__ void keys_kernel(const float4* __restrict__ in, uint64_t n, KeyGrid g
   vals[i] = (uint32_t)i;
 }
 
-// ---------------- stable LSD radix sort, 8-bit digits ----------------------
+// ---------------- stable LSD radix sort, 8- to 10-bit digits ----------------
 constexpr int kSortThreads = 256;
 constexpr int kSortItems = 8;
 constexpr int kSortTile = kSortThreads * kSortItems;  // 2048 keys per tile
 constexpr int kWarps = kSortThreads / 32;
 
 // Per-tile digit histogram, stored digit-major: hist[digit * tiles + tile].
+template <int kBits>
 __global__ void radix_hist_kernel(const uint32_t* __restrict__ keys, uint64_t n, int shift,
                                   uint32_t tiles, uint32_t* __restrict__ hist) {
-  __shared__ uint32_t h[256];
-  h[threadIdx.x] = 0;
+  constexpr int kBins = 1 << kBits;
+  __shared__ uint32_t h[kBins];
+  for (int d = threadIdx.x; d < kBins; d += kSortThreads) h[d] = 0;
   __syncthreads();
   const uint64_t base = (uint64_t)blockIdx.x * kSortTile;
 #pragma unroll
   for (int it = 0; it < kSortItems; ++it) {
     const uint64_t i = base + (uint64_t)it * kSortThreads + threadIdx.x;
-    if (i < n) atomicAdd(&h[(keys[i] >> shift) & 255u], 1u);
+    if (i < n) atomicAdd(&h[(keys[i] >> shift) & (kBins - 1u)], 1u);
   }
   __syncthreads();
-  hist[(uint64_t)threadIdx.x * tiles + blockIdx.x] = h[threadIdx.x];
+  for (int d = threadIdx.x; d < kBins; d += kSortThreads)
+    hist[(uint64_t)d * tiles + blockIdx.x] = h[d];
 }
 
 // Exclusive scan of m entries by one block of 1024 threads (chunked).
@@ -248,15 +266,18 @@ int scan_u32(uint32_t* a, uint64_t m, uint32_t* sums, cudaStream_t st) {
 // Stable scatter: items of a tile are ranked in index order (warp-contiguous
 // chunks of 256, lane-striped), per digit, then placed at the tile's scanned
 // digit offset.
+template <int kBits>
 __global__ void radix_scatter_kernel(const uint32_t* __restrict__ kin,
                                      const uint32_t* __restrict__ vin, uint64_t n, int shift,
                                      uint32_t tiles, const uint32_t* __restrict__ hist,
                                      uint32_t* __restrict__ kout, uint32_t* __restrict__ vout) {
-  __shared__ uint32_t wcount[kWarps][256];
-  __shared__ uint32_t goff[256];
+  constexpr int kBins = 1 << kBits;
+  __shared__ uint32_t wcount[kWarps][kBins];
+  __shared__ uint32_t goff[kBins];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int i = threadIdx.x; i < kWarps * 256; i += kSortThreads) (&wcount[0][0])[i] = 0;
-  goff[threadIdx.x] = hist[(uint64_t)threadIdx.x * tiles + blockIdx.x];
+  for (int i = threadIdx.x; i < kWarps * kBins; i += kSortThreads) (&wcount[0][0])[i] = 0;
+  for (int d = threadIdx.x; d < kBins; d += kSortThreads)
+    goff[d] = hist[(uint64_t)d * tiles + blockIdx.x];
   __syncthreads();
   const uint64_t base = (uint64_t)blockIdx.x * kSortTile + (uint64_t)warp * (32 * kSortItems);
   uint32_t k[kSortItems], v[kSortItems], rank[kSortItems];
@@ -267,7 +288,7 @@ __global__ void radix_scatter_kernel(const uint32_t* __restrict__ kin,
     const bool ok = i < n;
     k[it] = ok ? kin[i] : 0u;
     v[it] = ok ? vin[i] : 0u;
-    const unsigned digit = ok ? ((k[it] >> shift) & 255u) : (256u + lane);
+    const unsigned digit = ok ? ((k[it] >> shift) & (kBins - 1u)) : (kBins + lane);
     const unsigned peers = __match_any_sync(0xffffffffu, digit);
     const unsigned before = __popc(peers & lt);
     const unsigned leader = __ffs(peers) - 1;
@@ -279,8 +300,8 @@ __global__ void radix_scatter_kernel(const uint32_t* __restrict__ kin,
     __syncwarp();
   }
   __syncthreads();
-  {  // per digit: counts -> exclusive offsets across warps
-    const int d = threadIdx.x;
+  // per digit: counts -> exclusive offsets across warps
+  for (int d = threadIdx.x; d < kBins; d += kSortThreads) {
     uint32_t run = 0;
 #pragma unroll
     for (int w = 0; w < kWarps; ++w) {
@@ -294,7 +315,7 @@ __global__ void radix_scatter_kernel(const uint32_t* __restrict__ kin,
   for (int it = 0; it < kSortItems; ++it) {
     const uint64_t i = base + (uint64_t)it * 32 + lane;
     if (i < n) {
-      const unsigned digit = (k[it] >> shift) & 255u;
+      const unsigned digit = (k[it] >> shift) & (kBins - 1u);
       const uint32_t pos = goff[digit] + wcount[warp][digit] + rank[it];
       kout[pos] = k[it];
       vout[pos] = v[it];
@@ -302,40 +323,15 @@ __global__ void radix_scatter_kernel(const uint32_t* __restrict__ kin,
   }
 }
 
-// grid3d_sort_particles_into_cells + sorted->unsorted map
-__global__ void gather_kernel(const float4* __restrict__ in, const uint32_t* __restrict__ perm,
-                              uint64_t n, float4* __restrict__ out, uint32_t* __restrict__ s2u) {
-  const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const uint32_t j = perm[i];
-  out[i] = in[j];
-  s2u[i] = j;
-}
-
-// grid3d_determine_cells_begin / _end on the sorted keys
-__global__ void cell_ranges_kernel(const uint32_t* __restrict__ sk, uint64_t n,
-                                   int2* __restrict__ cells) {
-  const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const uint32_t k = sk[i];
-  if (i == 0 || sk[i - 1] != k) cells[k].x = (int)i;
-  if (i + 1 == n || sk[i + 1] != k) cells[k].y = (int)(i + 1);
-}
-
-// Sub-box code of every sorted particle: which sixteenth of its cell it lies in
-// per axis (clamped to 0..15), packed sx + 32 sy + 1024 sz (a free bit above
-// each field, for range tests by subtraction). The list builds use it only to
-// skip candidates that lie, by more than a rounding margin, outside the cube
-// of the current threshold around a point: those could never be inserted, so
-// skipping them leaves every result unchanged.
-__global__ void codes_kernel(const float4* __restrict__ parts, const uint32_t* __restrict__ sk,
-                             uint64_t n, KeyGrid kg, uint16_t* __restrict__ codes) {
-  const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const uint32_t k = sk[i];
-  const uint32_t kx = k % (uint32_t)kg.n0, kyz = k / (uint32_t)kg.n0;
+// Sub-box code of a particle: which sixteenth of its cell it lies in per axis
+// (clamped to 0..15), packed sx + 32 sy + 1024 sz (a free bit above each field,
+// for range tests by subtraction). The searches use it only to skip candidates
+// that lie, by more than a rounding margin, outside the cube of the current
+// threshold around a point: those could never be inserted, so skipping them
+// leaves every result unchanged.
+__device__ __forceinline__ uint16_t sub_box_code(const KeyGrid& kg, uint32_t key, const float4& p) {
+  const uint32_t kx = key % (uint32_t)kg.n0, kyz = key / (uint32_t)kg.n0;
   const uint32_t ky = kyz % (uint32_t)kg.n1, kz = kyz / (uint32_t)kg.n1;
-  const float4 p = parts[i];
   const float c[3] = {p.x, p.y, p.z};
   const float mn[3] = {kg.min0 + (float)kx * kg.cs0, kg.min1 + (float)ky * kg.cs1,
                        kg.min2 + (float)kz * kg.cs2};
@@ -346,11 +342,59 @@ __global__ void codes_kernel(const float4* __restrict__ parts, const uint32_t* _
     const float t = (c[a] - mn[a]) * iw[a];
     q[a] = t > 0.0f ? min((int)t, 15) : 0;
   }
-  codes[i] = (uint16_t)(q[0] | (q[1] << 5) | (q[2] << 10));
+  return (uint16_t)(q[0] | (q[1] << 5) | (q[2] << 10));
+}
+
+// After the sort, in one pass over the particles: the float4 records in cell
+// order with the sorted->unsorted map (grid3d_sort_particles_into_cells), the
+// cells' [begin, end) over a zeroed cell array (grid3d_determine_cells_begin /
+// _end) and, where codes is not null, the sub-box codes. Bound by the gather's
+// 32-byte sectors; three kernels that read the records and the keys again took
+// 25 us for 1,000,003 particles.
+__global__ void finish_kernel(const float4* __restrict__ in, const uint32_t* __restrict__ perm,
+                              const uint32_t* __restrict__ sk, uint64_t n, KeyGrid kg,
+                              float4* __restrict__ out, uint32_t* __restrict__ s2u,
+                              int2* __restrict__ cells, uint16_t* __restrict__ codes) {
+  const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const uint32_t j = perm[i], k = sk[i];
+  const float4 p = in[j];
+  if (i == 0 || sk[i - 1] != k) cells[k].x = (int)i;
+  if (i + 1 == n || sk[i + 1] != k) cells[k].y = (int)(i + 1);
+  out[i] = p;
+  s2u[i] = j;
+  if (codes) codes[i] = sub_box_code(kg, k, p);
 }
 
 inline unsigned grid_blocks(uint64_t n, int threads) {
   return (unsigned)((n + threads - 1) / threads);
+}
+
+}  // namespace
+
+namespace {
+
+// One pass over kBits bits of the keys from `shift` on. hist: tiles << kBits
+// counts, then the scan's chunk sums. Returns the kernels launched.
+template <int kBits>
+int radix_pass(const uint32_t* ka, const uint32_t* va, uint64_t n, int shift, uint32_t* hist,
+               uint32_t* kb, uint32_t* vb, cudaStream_t st) {
+  const uint64_t tiles = (n + kSortTile - 1) / kSortTile;
+  radix_hist_kernel<kBits><<<(unsigned)tiles, kSortThreads, 0, st>>>(ka, n, shift,
+                                                                     (uint32_t)tiles, hist);
+  const int scans = scan_u32(hist, tiles << kBits, hist + (tiles << kBits), st);
+  radix_scatter_kernel<kBits><<<(unsigned)tiles, kSortThreads, 0, st>>>(
+      ka, va, n, shift, (uint32_t)tiles, hist, kb, vb);
+  return 2 + scans;
+}
+
+// Bits of a digit: 8, or up to 10 where that saves a pass (keys of 17 to 20
+// bits: grids of 131,073 to 1,048,576 cells) and the histogram stays small.
+// Sorting 1,000,003 keys of 17 bits takes 2 passes of 36 us instead of 3.
+int digit_bits(int bits, uint64_t n) {
+  const int p8 = (bits + 7) / 8, p10 = (bits + 9) / 10;
+  if (p10 == p8 || n > (1ull << 23)) return 8;
+  return std::max(8, (bits + p10 - 1) / p10);
 }
 
 }  // namespace
@@ -362,7 +406,7 @@ cudaError_t grid_bbox(Context& c, const float4* in, uint64_t n, float* mn3, floa
   unsigned init[8] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0u, 0u, 0u, 0u, 0u};
   e = cudaMemcpyAsync(c.hist.p, init, sizeof(init), cudaMemcpyHostToDevice, c.stream);
   if (e) return e;
-  const unsigned blocks = (unsigned)std::min<uint64_t>(grid_blocks(n, 256), 148 * 8);
+  const unsigned blocks = (unsigned)std::min<uint64_t>(grid_blocks(n, 256), 148 * 4);
   bbox_kernel<<<blocks, 256, 0, c.stream>>>(in, n, c.hist.as<unsigned>());
   ++c.launches;
   e = cudaGetLastError();
@@ -405,10 +449,12 @@ cudaError_t grid_build_device(Context& c, const float4* in, uint64_t n) {
       (e = c.codes.ensure((n + 512) * 2)) || (e = c.cells.ensure(g.total * 8)) ||
       (e = c.flags.ensure(kFlagsBytes)))
     return e;
-  const uint64_t tiles = (n + kSortTile - 1) / kSortTile;
+  int bits = 1;
+  while (bits < 32 && (1ull << bits) < g.total) ++bits;
+  const int digit = digit_bits(bits, n);
   // histogram, then the scan's chunk sums
-  if ((e = c.hist.ensure(tiles * 256 * 4 + 4 * scan_chunks(tiles * 256) + 64))) return e;
-  uint32_t* chunk_sums = c.hist.as<uint32_t>() + tiles * 256;
+  const uint64_t counts = ((n + kSortTile - 1) / kSortTile) << digit;
+  if ((e = c.hist.ensure(counts * 4 + 4 * scan_chunks(counts) + 64))) return e;
   if ((e = cudaMemsetAsync(c.flags.p, 0, kFlagsBytes, c.stream))) return e;
 
   KeyGrid kg{g.min[0], g.min[1], g.min[2], g.cs[0], g.cs[1], g.cs[2], g.n[0], g.n[1], g.total};
@@ -417,28 +463,21 @@ cudaError_t grid_build_device(Context& c, const float4* in, uint64_t n) {
                                                           c.flags.as<uint32_t>());
   if ((e = cudaGetLastError())) return e;
 
-  int bits = 1;
-  while (bits < 32 && (1ull << bits) < g.total) ++bits;
   uint32_t *ka = c.keys_a.as<uint32_t>(), *kb = c.keys_b.as<uint32_t>();
   uint32_t *va = c.vals_a.as<uint32_t>(), *vb = c.vals_b.as<uint32_t>();
-  for (int shift = 0; shift < bits; shift += 8) {
-    radix_hist_kernel<<<(unsigned)tiles, kSortThreads, 0, c.stream>>>(
-        ka, n, shift, (uint32_t)tiles, c.hist.as<uint32_t>());
-    c.launches += 2 + scan_u32(c.hist.as<uint32_t>(), tiles * 256, chunk_sums, c.stream);
-    radix_scatter_kernel<<<(unsigned)tiles, kSortThreads, 0, c.stream>>>(
-        ka, va, n, shift, (uint32_t)tiles, c.hist.as<uint32_t>(), kb, vb);
+  const auto pass = digit == 10 ? radix_pass<10> : digit == 9 ? radix_pass<9> : radix_pass<8>;
+  for (int shift = 0; shift < bits; shift += digit) {
+    c.launches += pass(ka, va, n, shift, c.hist.as<uint32_t>(), kb, vb, c.stream);
     if ((e = cudaGetLastError())) return e;
     std::swap(ka, kb);
     std::swap(va, vb);
   }
-  gather_kernel<<<grid_blocks(n, 256), 256, 0, c.stream>>>(in, va, n, c.parts.as<float4>(),
-                                                            c.s2u.as<uint32_t>());
   c.sorted_keys = ka;
   if ((e = cudaMemsetAsync(c.cells.p, 0, g.total * 8, c.stream))) return e;
-  cell_ranges_kernel<<<grid_blocks(n, 256), 256, 0, c.stream>>>(ka, n, c.cells.as<int2>());
-  codes_kernel<<<grid_blocks(n, 256), 256, 0, c.stream>>>(c.parts.as<float4>(), ka, n, kg,
-                                                           c.codes.as<uint16_t>());
-  c.launches += 4;  // keys, gather, cell ranges, codes
+  finish_kernel<<<grid_blocks(n, 256), 256, 0, c.stream>>>(
+      in, va, ka, n, kg, c.parts.as<float4>(), c.s2u.as<uint32_t>(), c.cells.as<int2>(),
+      c.codes.as<uint16_t>());
+  c.launches += 2;  // keys, finish
   return cudaGetLastError();
 }
 
@@ -534,7 +573,7 @@ extern "C" ilc_status ilc_grid_build_noalloc(const float* particles, uint64_t n,
   if (cudaMemcpyAsync(acc, init, sizeof(init), cudaMemcpyHostToDevice, st) != cudaSuccess ||
       cudaMemsetAsync(flags, 0, 64, st) != cudaSuccess)
     return ILC_ERR_CUDA;
-  bbox_kernel<<<(unsigned)std::min<uint64_t>(grid_blocks(n, 256), 148 * 8), 256, 0, st>>>(in, n,
+  bbox_kernel<<<(unsigned)std::min<uint64_t>(grid_blocks(n, 256), 148 * 4), 256, 0, st>>>(in, n,
                                                                                          acc);
   unsigned box[8];
   if (cudaGetLastError() != cudaSuccess ||
@@ -586,19 +625,18 @@ extern "C" ilc_status ilc_grid_build_noalloc(const float* particles, uint64_t n,
   int bits = 1;
   while (bits < 32 && (1ull << bits) < total) ++bits;
   for (int shift = 0; shift < bits; shift += 8) {
-    radix_hist_kernel<<<(unsigned)tiles, kSortThreads, 0, st>>>(ka, n, shift, (uint32_t)tiles,
-                                                                 hist);
+    radix_hist_kernel<8><<<(unsigned)tiles, kSortThreads, 0, st>>>(ka, n, shift,
+                                                                    (uint32_t)tiles, hist);
     scan_kernel<<<1, 1024, 0, st>>>(hist, tiles * 256);
-    radix_scatter_kernel<<<(unsigned)tiles, kSortThreads, 0, st>>>(ka, va, n, shift,
-                                                                   (uint32_t)tiles, hist, kb, vb);
+    radix_scatter_kernel<8><<<(unsigned)tiles, kSortThreads, 0, st>>>(
+        ka, va, n, shift, (uint32_t)tiles, hist, kb, vb);
     std::swap(ka, kb);
     std::swap(va, vb);
   }
-  gather_kernel<<<grid_blocks(n, 256), 256, 0, st>>>(in, va, n,
-                                                      reinterpret_cast<float4*>(sorted_particles),
-                                                      sorted_to_unsorted);
   if (cudaMemsetAsync(cells, 0, total * 8, st) != cudaSuccess) return ILC_ERR_CUDA;
-  cell_ranges_kernel<<<grid_blocks(n, 256), 256, 0, st>>>(ka, n, reinterpret_cast<int2*>(cells));
+  finish_kernel<<<grid_blocks(n, 256), 256, 0, st>>>(
+      in, va, ka, n, kg, reinterpret_cast<float4*>(sorted_particles), sorted_to_unsorted,
+      reinterpret_cast<int2*>(cells), nullptr);
   uint32_t f = 0;
   if (cudaGetLastError() != cudaSuccess ||
       cudaMemcpyAsync(&f, flags, 4, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
