@@ -287,7 +287,7 @@ adjoint_kernel(const __grid_constant__ AdjK a, const __grid_constant__ GridView 
     const float zq = step_point(z, h, pj);
     PointSlots s;
     eval_points<true>(g, M.spiral, W, lane, go && !(replay && pj == 3), px, py, pz, lx,
-                               ly, lz, zq, s, ws);
+                               ly, lz, zq, h, s, ws);
     ScatterSlots cur;
     if (go) scatter_slots(s, cur);
     bool accepted = go;
@@ -417,7 +417,9 @@ cudaError_t adjoint_ray_launch(Context& c, const RenderArgs& r, int mode, const 
                                                          sizeof(AdjMem))))
     return e;
   const unsigned long long resident = (unsigned long long)sms * (per_sm > 0 ? per_sm : 1);
-  const unsigned blocks = (unsigned)(resident < 4 * tiles ? resident : 4 * tiles);
+  // (down to one ray per warp)
+  const unsigned long long most = 128 / kListWarps * tiles;
+  const unsigned blocks = (unsigned)(resident < most ? resident : most);
   if ((e = c.list_over.ensure((size_t)blocks * kListWarps * kRays * kOver * 16))) return e;
   k.over = c.list_over.as<float4>();
   if (!c.ev0) {

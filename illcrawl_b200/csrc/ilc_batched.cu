@@ -250,7 +250,7 @@ batched_kernel(const __grid_constant__ BatchK a, const __grid_constant__ GridVie
       if (pj == 0) atomicAdd(&M.stats[6], 1ull);
       go = false;
     }
-    eval_points<kMulti>(g, M.spiral, W, lane, go, ox, oy, oz, lx, ly, lz, zq, s, ws);
+    eval_points<kMulti>(g, M.spiral, W, lane, go, ox, oy, oz, lx, ly, lz, zq, h, s, ws);
     if (!kMulti) {
       float e[4];
       share4(go ? slots_value(s) : 0.0f, lane, e);

@@ -181,6 +181,28 @@ __device__ __forceinline__ void nn8_walk(const GridView& g, const char4* __restr
   }
 }
 
+// 1 / b and sqrt(x), correctly rounded, without branches, for arguments well
+// inside the normal range: Newton steps on the hardware's approximations with
+// Markstein's final correction ("IA-64 and Elementary Functions", 2000, chapters
+// 8 and 9). Compared with the IEEE operations for every significand (both
+// exponent parities for the root): no difference.
+__device__ __forceinline__ float rcp_normal(float b) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));
+  return __fmaf_rn(__fmaf_rn(-b, y, 1.0f), y, y);
+}
+__device__ __forceinline__ float sqrt_normal(float x) {
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  float g = x * y, h = 0.5f * y;
+  const float r = __fmaf_rn(-h, g, 0.5f);
+  g = __fmaf_rn(g, r, g);
+  h = __fmaf_rn(h, r, h);
+  return __fmaf_rn(__fmaf_rn(-g, g, x), h, g);
+}
+// Range of squared distances for both (and for 1 / d^2).
+__device__ __forceinline__ bool plain_d2(float d2) { return d2 >= 1e-30f && d2 <= 1e30f; }
+
 // get_weight3d + finalize (volumetric_nn8_reconstruction.cl:44-50,212-270)
 __device__ __forceinline__ float weight3d(float d) {
   const float i2 = 1.0f / (d * d);

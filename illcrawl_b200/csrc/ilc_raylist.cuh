@@ -134,7 +134,7 @@ struct BuildState {
 
 __device__ __forceinline__ void build_radius(BuildState& b, int lane) {
   b.R2 = __uint_as_float(__reduce_max_sync(kAll, lane < 8 ? __float_as_uint(b.s8) : 0u));
-  b.R = sqrtf(b.R2);
+  asm("sqrt.approx.f32 %0, %1;" : "=f"(b.R) : "f"(b.R2));  // (within the slack of T)
   b.T = (b.R + b.tb) * 1.00001f;
   b.T2 = b.T * b.T;
 }
@@ -480,9 +480,11 @@ __device__ __forceinline__ int build_list(const GridView& g, const char4* __rest
   return tested;
 }
 
-// A lane's slots after its point's walk: distances and values (indices).
+// A lane's slots after its point's walk: distances and values (indices);
+// plain: every squared distance is plain_d2.
 struct PointSlots {
   float d[8], v[8];
+  bool plain;
 };
 
 __device__ __forceinline__ float max8(const float d[8]) {
@@ -581,20 +583,30 @@ __device__ __forceinline__ void replay_point(const GridView& g, const WarpLists&
     for (int q = 0; q < 8; ++q)
       o.v[q] = o.d[q] < FLT_MAX ? list_entry(W, r, ix[q]).w : (kIdx ? __int_as_float(-1) : 0.0f);
   }
+  o.plain = false;
   if (!exact) {
+    float lo = fminf(o.d[0], o.d[1]);
 #pragma unroll
-    for (int q = 0; q < 8; ++q) o.d[q] = sqrtf(o.d[q]);
+    for (int q = 2; q < 8; ++q) lo = fminf(lo, o.d[q]);
+    o.plain = plain_d2(lo) && plain_d2(max8(o.d));
+    if (o.plain) {
+#pragma unroll
+      for (int q = 0; q < 8; ++q) o.d[q] = sqrt_normal(o.d[q]);
+    } else {
+#pragma unroll
+      for (int q = 0; q < 8; ++q) o.d[q] = sqrtf(o.d[q]);
+    }
   }
 }
 
 // nn8 slots of the lanes' points: lane 4r + j holds point j of ray r at
-// position (x, y, z) = o + zq l. `active` lanes get their slots. The whole
-// warp calls this together.
+// position (x, y, z) = o + zq l, h the ray's step. `active` lanes get their
+// slots. The whole warp calls this together.
 template <bool kIdx>
 __device__ __forceinline__ void eval_points(const GridView& g, const char4* __restrict__ spiral,
                                             WarpLists& W, int lane, bool active, float ox,
                                             float oy, float oz, float lx, float ly, float lz,
-                                            float zq, PointSlots& o, WalkStats& st) {
+                                            float zq, float h, PointSlots& o, WalkStats& st) {
   const float x = ox + zq * lx, y = oy + zq * ly, z = oz + zq * lz;
   const int r = lane >> 2;
   const unsigned mine = 0xfu << (lane & 28);
@@ -636,7 +648,7 @@ __device__ __forceinline__ void eval_points(const GridView& g, const char4* __re
                     roz = __shfl_sync(kAll, oz, lead);
         const float rlx = __shfl_sync(kAll, lx, lead), rly = __shfl_sync(kAll, ly, lead),
                     rlz = __shfl_sync(kAll, lz, lead);
-        const float zl = __shfl_sync(kAll, zq, lead);
+        const float zl = __shfl_sync(kAll, zq, lead), hl = __shfl_sync(kAll, h, lead);
         // finite positions only: anything else is walked by one thread
         const bool fin = fabsf(x) < 1e15f && fabsf(y) < 1e15f && fabsf(z) < 1e15f &&
                          fabsf(zq) < 1e15f;
@@ -684,13 +696,21 @@ __device__ __forceinline__ void eval_points(const GridView& g, const char4* __re
             if (tested >= 0) break;
             ext *= 0.6f;
           }
-          // longer lists pay where the search behind them is long
           ok = tested >= 0;
           if (ok) {
-            const int n = W.meta[lr].n, want = tested > 256 ? 62 : 34;
-            const int nu = W.meta[lr].nu;
-            if (n > want || nu > kUnc - 4) ext *= 0.85f;
-            else if (n < want - 8 && nu < kUnc - 8) ext *= 1.2f;
+            const int n = W.meta[lr].n, nu = W.meta[lr].nu;
+            // The cost per step is least where a build's share of it equals
+            // what its length adds to each replay. In warp instructions: a
+            // build takes about 500, 0.4 per candidate looked at and 30 per
+            // candidate kept; a candidate or break cell beyond the 16 of a
+            // point's own list 14 of a replay. (6 / 12 / 24 for the 14:
+            // projection 348 / 335 / 347 ms, 2048 fixed steps 151 / 128 / 133
+            // ms, tilted band map through a core 37 / 35 / 33 ms; a fixed aim
+            // of 34 candidates, 62 behind long searches: 418 / 151 / 45 ms.)
+            const float build = (500.0f + 0.4f * (float)tested + 30.0f * (float)n) * hl;
+            const float replay = 14.0f * (float)(n + nu - 16) * (b - a);
+            if (build < 0.8f * replay || nu > kUnc - 3 || n > 200) ext *= 0.85f;
+            else if (build > 1.25f * replay) ext *= 1.2f;
           }
           ext = fminf(fmaxf(ext, g.half0 * 1e-4f), g.cs0);
           __syncwarp();
@@ -710,6 +730,7 @@ __device__ __forceinline__ void eval_points(const GridView& g, const char4* __re
             }
             W.meta[lr].za = 1.0f;
             W.meta[lr].zb = 0.0f;
+            o.plain = false;
             todo = false;
           }
           __syncwarp();
@@ -732,8 +753,17 @@ __device__ __forceinline__ void eval_points(const GridView& g, const char4* __re
 // get_weight3d and finalize in slot order
 // (volumetric_nn8_reconstruction.cl:44-50,212-270).
 __device__ __forceinline__ void slot_weights(const PointSlots& s, float w[8], float& ws) {
+  if (s.plain) {
 #pragma unroll
-  for (int t = 0; t < 8; ++t) w[t] = weight3d(s.d[t]);
+    for (int t = 0; t < 8; ++t) {
+      const float i2 = rcp_normal(s.d[t] * s.d[t]);
+      const float i4 = i2 * i2;
+      w[t] = (i4 * i4) * i2;
+    }
+  } else {
+#pragma unroll
+    for (int t = 0; t < 8; ++t) w[t] = weight3d(s.d[t]);
+  }
   ws = 0.0f;
 #pragma unroll
   for (int t = 0; t < 8; ++t) ws = ws + w[t];

@@ -158,7 +158,7 @@ render_kernel(const __grid_constant__ RenderK a, const __grid_constant__ GridVie
     if (go && a.replay_h) h = hs[steps];
     const float zq = step_point(z, h, pj);
     PointSlots s;
-    eval_points<false>(g, M.spiral, W, lane, go, px, py, pz, lx, ly, lz, zq, s, ws);
+    eval_points<false>(g, M.spiral, W, lane, go, px, py, pz, lx, ly, lz, zq, h, s, ws);
     float e[4];
     share4(go ? slots_value(s) : 0.0f, lane, e);
     if (go) {
@@ -284,9 +284,11 @@ cudaError_t render_launch(Context& c, const RenderArgs& a, float* kernel_ms) {
                                                          sizeof(RenderMem))))
     return e;
   if (occ > 0) per_sm = std::min(per_sm, occ);
+  // (down to one ray per warp: the rays of a small image build and replay their
+  // lists next to each other instead of in turn)
   const unsigned blocks =
       (unsigned)std::min<unsigned long long>((unsigned long long)sms * std::max(per_sm, 1),
-                                             4 * tiles);
+                                             128 / kListWarps * tiles);
   if ((e = c.list_over.ensure((size_t)blocks * kListWarps * kRays * kOver * 16))) return e;
   k.over = c.list_over.as<float4>();
   if (!c.ev0) {
