@@ -39,12 +39,14 @@
 // lanes replay (a list holds 14-28 candidates, 5 break cells are passed), and
 // a cell of 20,000 candidates is scanned 256 at a time. Measured on a B200,
 // before -> after: band map of the outer 1.5 Mpc slab of 4,194,304 cells,
-// 256^2: 600 -> 250 ms; projection of 262,144 cells, 256^2, 3 Mpc: 1,450 ->
-// 472 ms; 101 x 75 tilted band map through the core of 1 M cells: 1,570 ->
-// 45 ms; 2048 fixed steps, 200^2: 327 -> 184 ms; 128-bin spectra of three
-// cameras: 942 -> 45 ms; adjoint of a 64^2 band map: 1,413 -> 211 ms. Bound by
-// instruction issue and shared-memory latency of the replays; the grid stays
-// in L2.
+// 256^2: 600 -> 197 ms; projection of 262,144 cells, 256^2, 3 Mpc: 1,450 ->
+// 292 ms; 101 x 75 tilted band map through the core of 1 M cells: 1,570 ->
+// 34 ms; 2048 fixed steps, 200^2: 327 -> 128 ms; 128-bin spectra of three
+// cameras: 942 -> 33 ms; adjoint of a 64^2 band map: 1,413 -> 88 ms. Bound by
+// instruction issue: 42 % of the slots, the rest instruction fetch (5,400
+// instructions of kernel, as much stall as dependent arithmetic) and the
+// latency of dependent arithmetic with 4 warps per scheduler; the grid stays in
+// L2 (DRAM 3 MB read per launch).
 #pragma once
 
 #include "ilc_device.cuh"
@@ -53,8 +55,8 @@ namespace ilc {
 
 constexpr int kRays = 8;             // rays of a warp
 constexpr int kUnc = 20;             // cells a list's points may break at
-constexpr int kCap = 64;             // candidates of a list in shared memory
-constexpr int kOver = 191;           // and further ones in global memory (dense cores)
+constexpr int kCap = 48;             // candidates of a list in shared memory
+constexpr int kOver = 207;           // and further ones in global memory (dense cores)
 constexpr int kCapAll = kCap + kOver;  // 255: positions fit a byte
 constexpr int kHits = 96;            // build: buffered hits of the sub-box codes
 constexpr int kListThreads = 128;    // threads of a block: 4 warps, 32 rays
@@ -709,7 +711,12 @@ __device__ __forceinline__ void eval_points(const GridView& g, const char4* __re
             // of 34 candidates, 62 behind long searches: 418 / 151 / 45 ms.)
             const float build = (500.0f + 0.4f * (float)tested + 30.0f * (float)n) * hl;
             const float replay = 14.0f * (float)(n + nu - 16) * (b - a);
-            if (build < 0.8f * replay || nu > kUnc - 3 || n > 200) ext *= 0.85f;
+            // (Break cells near the limit, where a build is lost, shorten it at
+            // once: projection 337 -> 292 ms, adjoint of a 64^2 map 108 -> 85
+            // ms, with 48 instead of 64 candidates in shared memory, which
+            // leaves 70 KB of L1 for the grid.)
+            if (nu > kUnc - 6) ext *= 0.6f;
+            else if (build < 0.8f * replay || n > 200) ext *= 0.85f;
             else if (build > 1.25f * replay) ext *= 1.2f;
           }
           ext = fminf(fmaxf(ext, g.half0 * 1e-4f), g.cs0);
