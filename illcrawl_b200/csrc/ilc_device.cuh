@@ -203,34 +203,11 @@ __device__ __forceinline__ float sqrt_normal(float x) {
 // Range of squared distances for both (and for 1 / d^2).
 __device__ __forceinline__ bool plain_d2(float d2) { return d2 >= 1e-30f && d2 <= 1e30f; }
 
-// get_weight3d + finalize (volumetric_nn8_reconstruction.cl:44-50,212-270)
+// get_weight3d (volumetric_nn8_reconstruction.cl:44-50)
 __device__ __forceinline__ float weight3d(float d) {
   const float i2 = 1.0f / (d * d);
   const float i4 = i2 * i2;
   return (i4 * i4) * i2;
-}
-
-template <bool kIds> __device__ __forceinline__ float nn8_finalize(const Slots<kIds>& s) {
-  float w[8];
-#pragma unroll
-  for (int j = 0; j < 8; ++j) w[j] = weight3d(s.d[j]);
-  float ws = 0.0f;
-#pragma unroll
-  for (int j = 0; j < 8; ++j) ws = ws + w[j];
-  float dot = 0.0f;
-#pragma unroll
-  for (int j = 0; j < 8; ++j) dot = __fmaf_rn(w[j], s.v[j], dot);
-  float res = 0.0f;
-  if (ws != 0.0f && dot != 0.0f) res = dot / ws;
-  return res;
-}
-
-__device__ __forceinline__ float nn8_value(const GridView& g, const char4* spiral, float x,
-                                           float y, float z, WalkStats& st) {
-  Slots<false> s;
-  s.init();
-  nn8_walk<false>(g, spiral, x, y, z, s, st);
-  return nn8_finalize(s);
 }
 
 // Copies the 8 x 125 spiral table into shared memory (block-wide).

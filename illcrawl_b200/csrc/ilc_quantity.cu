@@ -159,11 +159,12 @@ xray_bin_kernel(const float* __restrict__ table, const __grid_constant__ GauntVi
 // (the quantity of each frame of spectrum_generator, spectrum.cpp:89-109, or
 // of chandra_spectrum_quantity_generator, spectrum.cpp:45-65).
 //
-// A warp takes 32 cells: each lane prepares one of them in shared memory, then
-// the lanes run over the 32 x n_bins outputs, which are consecutive in memory.
+// A warp takes `group` cells (at most 32): each lane prepares one of them in
+// shared memory, then the lanes run over the group x n_bins outputs, which are
+// consecutive in memory.
 // So what depends on the cell is computed once instead of once per bin, and
 // what depends on the bin once per block and chunk of bins. 128 bins of 300,007
-// cells: 592 -> 270 us; 3 blocks per SM (71 registers, 75 KB).
+// cells: 592 -> 256 us; 3 blocks per SM (71 registers, 66 KB).
 constexpr int kBinChunk = 128;
 struct CellShare {
   EmitCell c;
@@ -176,14 +177,15 @@ bins_kernel(const float* __restrict__ table, const __grid_constant__ GauntView G
             const float* __restrict__ arf, ArfView A, const float* __restrict__ rho,
             const float* __restrict__ u, const float* __restrict__ xe, uint64_t n, float z,
             float dL, const float* __restrict__ e, const float* __restrict__ de, int n_bins,
-            float* __restrict__ out) {
+            int group, float* __restrict__ out) {
   extern __shared__ __align__(16) float t[];
   Channel* ch = reinterpret_cast<Channel*>(t + kTableFloats);
   CellShare* cells = reinterpret_cast<CellShare*>(ch + kBinChunk) + (threadIdx.x & ~31u);
   load_table(t, table, (G.w + 2 * G.pad) * (G.h + 2 * G.pad));
   const EmitCall k = emit_call(G, dL);
   const int lane = threadIdx.x & 31;
-  const uint64_t groups = (n + 31) / 32, warps = (uint64_t)gridDim.x * (kThreads / 32);
+  const uint64_t groups = (n + group - 1) / group;
+  const uint64_t warps = (uint64_t)gridDim.x * (kThreads / 32);
   const uint64_t w0 = first_group();
   for (int b0 = 0; b0 < n_bins; b0 += kBinChunk) {
     const int nb = min(kBinChunk, n_bins - b0);
@@ -192,8 +194,8 @@ bins_kernel(const float* __restrict__ table, const __grid_constant__ GauntView G
       ch[b] = make_channel<kChandra>(arf, A, e[b0 + b], de[b0 + b], z);
     __syncthreads();
     for (uint64_t g = w0; g < groups; g += warps) {
-      const uint64_t i0 = g * 32;
-      const int m = (int)min((uint64_t)32, n - i0);
+      const uint64_t i0 = g * group;
+      const int m = (int)min((uint64_t)group, n - i0);
       __syncwarp();
       if (lane < m) {
         CellShare s;
@@ -258,10 +260,10 @@ __global__ void temperature_kernel(const float* __restrict__ u, const float* __r
 // As many blocks as are resident (per_sm each), so that a block loads the
 // table once; fewer for a few cells. A block's warps take 32 cells each, dealt
 // over all blocks first, so that every SM gets its share of a few cells too.
-unsigned resident_blocks(const Context& c, uint64_t n, int per_sm) {
+unsigned resident_blocks(const Context& c, uint64_t groups, int per_sm) {
   int sms = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c.device);
-  const uint64_t want = (n + 31) / 32, fit = (uint64_t)(sms > 0 ? sms : 148) * per_sm;
+  const uint64_t want = groups, fit = (uint64_t)(sms > 0 ? sms : 148) * per_sm;
   return (unsigned)(want < fit ? want : fit);
 }
 
@@ -270,15 +272,28 @@ GauntView gaunt_view(const Context& c) {
 }
 ArfView arf_view(const Context& c) { return ArfView{c.arf_n, c.arf_x0, c.arf_dx}; }
 
-// Launches one of the kernels above with its dynamic shared memory.
+// Cells per warp of a bin table: enough for about 32 turns of its lanes, and
+// fewer, down to one, while that leaves warps without a group. (300,007 cells of
+// 128 bins: 268 us in groups of 32, 256 us in groups of 8; 300 cells of 128
+// bins: 52 us and 28 us, 34 us when every output was a thread of its own.)
+int bin_group(uint64_t n, int n_bins) {
+  int group = 32;
+  while (group > 1 && ((int64_t)group * n_bins > 1024 ||
+                       ((int64_t)group * n_bins > 32 && n / group < 148 * 3 * (kThreads / 32))))
+    group /= 2;
+  return group;
+}
+
+// Launches one of the kernels above, a warp to each of `groups`, with its
+// dynamic shared memory.
 template <class... P, class... Q>
-cudaError_t launch(Context& c, void (*kernel)(P...), uint64_t n, int per_sm, size_t smem,
+cudaError_t launch(Context& c, void (*kernel)(P...), uint64_t groups, int per_sm, size_t smem,
                    Q... args) {
   const cudaError_t e = cudaFuncSetAttribute(
       kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e) return e;
   ++c.launches;
-  kernel<<<resident_blocks(c, n, per_sm), kThreads, smem, c.stream>>>(
+  kernel<<<resident_blocks(c, groups, per_sm), kThreads, smem, c.stream>>>(
       c.gaunt_pad.as<float>(), gaunt_view(c), args...);
   return cudaGetLastError();
 }
@@ -290,7 +305,7 @@ cudaError_t quantity_xray_flux_launch(Context& c, const float* rho, const float*
                                       const float* xe, uint64_t n, float z, float dL,
                                       float emin, float emax, int num_samples, float* out,
                                       int out_stride) {
-  return launch(c, xray_flux_kernel<false>, n, kBlocksPerSm, kTableSmem, rho, u, xe, n, z, dL,
+  return launch(c, xray_flux_kernel<false>, (n + 31) / 32, kBlocksPerSm, kTableSmem, rho, u, xe, n, z, dL,
                 emin, emax, num_samples, out, out_stride);
 }
 
@@ -298,21 +313,21 @@ cudaError_t quantity_xray_photon_flux_launch(Context& c, const float* rho, const
                                              const float* xe, uint64_t n, float z, float dL,
                                              float emin, float emax, int num_samples,
                                              float* out) {
-  return launch(c, xray_flux_kernel<true>, n, kBlocksPerSm, kTableSmem, rho, u, xe, n, z, dL,
+  return launch(c, xray_flux_kernel<true>, (n + 31) / 32, kBlocksPerSm, kTableSmem, rho, u, xe, n, z, dL,
                 emin, emax, num_samples, out, 1);
 }
 
 cudaError_t quantity_chandra_total_launch(Context& c, const float* rho, const float* u,
                                           const float* xe, uint64_t n, float z, float dL,
                                           float* out) {
-  return launch(c, chandra_total_kernel, n, kBlocksPerSm, kTableSmem + kChunk * sizeof(Channel),
+  return launch(c, chandra_total_kernel, (n + 31) / 32, kBlocksPerSm, kTableSmem + kChunk * sizeof(Channel),
                 c.arf.as<float>(), arf_view(c), rho, u, xe, n, z, dL, out);
 }
 
 cudaError_t quantity_chandra_bin_launch(Context& c, const float* rho, const float* u,
                                         const float* xe, uint64_t n, float z, float dL, float e,
                                         float de, float* out) {
-  return launch(c, chandra_bin_kernel, n, kBlocksPerSm, kTableSmem, c.arf.as<float>(),
+  return launch(c, chandra_bin_kernel, (n + 31) / 32, kBlocksPerSm, kTableSmem, c.arf.as<float>(),
                 arf_view(c), rho, u, xe, n, z, dL, e, de, out);
 }
 
@@ -320,22 +335,24 @@ cudaError_t quantity_chandra_bins_launch(Context& c, const float* rho, const flo
                                          const float* xe, uint64_t n, float z, float dL,
                                          const float* e, const float* de, int n_bins,
                                          float* out) {
-  return launch(c, bins_kernel<true>, n, 3, kBinsSmem, c.arf.as<float>(), arf_view(c), rho, u, xe,
-                n, z, dL, e, de, n_bins, out);
+  const int group = bin_group(n, n_bins);
+  return launch(c, bins_kernel<true>, (n + group - 1) / group, 3, kBinsSmem, c.arf.as<float>(),
+                arf_view(c), rho, u, xe, n, z, dL, e, de, n_bins, group, out);
 }
 
 cudaError_t quantity_xray_bin_launch(Context& c, const float* rho, const float* u,
                                      const float* xe, uint64_t n, float z, float dL, float e,
                                      float de, float* out) {
-  return launch(c, xray_bin_kernel, n, kBlocksPerSm, kTableSmem, rho, u, xe, n, z, dL, e, de,
+  return launch(c, xray_bin_kernel, (n + 31) / 32, kBlocksPerSm, kTableSmem, rho, u, xe, n, z, dL, e, de,
                 out);
 }
 
 cudaError_t quantity_xray_bins_launch(Context& c, const float* rho, const float* u,
                                       const float* xe, uint64_t n, float z, float dL,
                                       const float* e, const float* de, int n_bins, float* out) {
-  return launch(c, bins_kernel<false>, n, 3, kBinsSmem, c.arf.as<float>(), arf_view(c), rho, u,
-                xe, n, z, dL, e, de, n_bins, out);
+  const int group = bin_group(n, n_bins);
+  return launch(c, bins_kernel<false>, (n + group - 1) / group, 3, kBinsSmem, c.arf.as<float>(),
+                arf_view(c), rho, u, xe, n, z, dL, e, de, n_bins, group, out);
 }
 
 cudaError_t quantity_temperature_launch(Context& c, const float* u, const float* xe,
