@@ -35,17 +35,19 @@
 // 770 warp instructions per step with 10 of 32 lanes active (band map of
 // 4,194,304 cells, 1 Mpc from the core), and a warp whose rays cross a dense
 // cell spent 100-600 us per step scanning it 16 candidates at a time in one
-// lane. Here a search is made once per ~10-20 steps by 32 lanes, 24 of 32
-// lanes replay (a list holds 14-28 candidates, 5 break cells are passed), and
-// a cell of 20,000 candidates is scanned 256 at a time. Measured on a B200,
+// lane. Here 32 lanes make a search for several steps, and a cell of 20,000
+// candidates is scanned 256 at a time. Counted on a B200 over six renders,
+// before list lengths followed their cost: one search per 6-19 steps, 14-28
+// candidates and 6-10 break cells per list, 22-25 of 32 lanes replaying in
+// sparse cells but 4-8 where core rays have a warp to themselves. Times there,
 // before -> after: band map of the outer 1.5 Mpc slab of 4,194,304 cells,
 // 256^2: 600 -> 197 ms; projection of 262,144 cells, 256^2, 3 Mpc: 1,450 ->
 // 292 ms; 101 x 75 tilted band map through the core of 1 M cells: 1,570 ->
 // 34 ms; 2048 fixed steps, 200^2: 327 -> 128 ms; 128-bin spectra of three
 // cameras: 942 -> 33 ms; adjoint of a 64^2 band map: 1,413 -> 88 ms. Bound by
-// instruction issue: 42 % of the slots, the rest instruction fetch (5,400
-// instructions of kernel, as much stall as dependent arithmetic) and the
-// latency of dependent arithmetic with 4 warps per scheduler; the grid stays in
+// instruction issue: 42 % of the slots, the rest the latency of dependent
+// arithmetic with 4 warps per scheduler (stalls of 2.6 cycles per issue) and
+// instruction fetch (1.9; 5,400 instructions of kernel); the grid stays in
 // L2 (DRAM 3 MB read per launch).
 #pragma once
 
