@@ -44,11 +44,15 @@
 // 256^2: 600 -> 197 ms; projection of 262,144 cells, 256^2, 3 Mpc: 1,450 ->
 // 292 ms; 101 x 75 tilted band map through the core of 1 M cells: 1,570 ->
 // 34 ms; 2048 fixed steps, 200^2: 327 -> 128 ms; 128-bin spectra of three
-// cameras: 942 -> 33 ms; adjoint of a 64^2 band map: 1,413 -> 88 ms. Bound by
-// instruction issue: 42 % of the slots, the rest the latency of dependent
-// arithmetic with 4 warps per scheduler (stalls of 2.6 cycles per issue) and
-// instruction fetch (1.9; 5,400 instructions of kernel); the grid stays in
-// L2 (DRAM 3 MB read per launch).
+// cameras: 942 -> 33 ms; adjoint of a 64^2 band map: 1,413 -> 85 ms. Bound by
+// instruction issue (44 % of the slots; small outer-slab band map), dependent
+// arithmetic with 4 warps per scheduler (stalls of 2.3 cycles per issue) and
+// instruction fetch (2.0); the grid stays in L2 (DRAM 2 MB read per launch).
+// Images of very many rays gain less, since there the walks from scratch filled
+// the chip too: 1024^2 band map of 4,194,304 cells, 6 Mpc: 12.16 -> 10.77 s; and
+// loose tolerances away from dense cores, whose steps are long, lose: 256^2 /
+// 1024^2 projection of 262,144 cells through the outer 500 kpc at rtol 1e-2:
+// 3.3 -> 5.6 / 19 -> 81 ms (through the core, 2 Mpc, 256^2: 554 -> 44 ms).
 #pragma once
 
 #include "ilc_device.cuh"
