@@ -30,12 +30,14 @@ struct QueryBins {
 
 __device__ __forceinline__ uint32_t query_bin(const GridView& g, const QueryBins& b,
                                               const float4& q) {
-  // (order only: nothing depends on the rounding here; NaN goes to 0)
+  // (order only: nothing depends on the rounding here; NaN goes to 0. The upper
+  // limit is an integer one: 2 n - 1 as a float is 2 n, a cell too far, on axes
+  // of more than 2^23 cells.)
   const float h0 = (q.x - g.min0) * (2.0f / g.cs0), h1 = (q.y - g.min1) * (2.0f / g.cs1),
               h2 = (q.z - g.min2) * (2.0f / g.cs2);
-  const uint32_t i0 = (uint32_t)fminf(fmaxf(h0, 0.0f), 2.0f * (float)b.n0 - 1.0f);
-  const uint32_t i1 = (uint32_t)fminf(fmaxf(h1, 0.0f), 2.0f * (float)b.n1 - 1.0f);
-  const uint32_t i2 = (uint32_t)fminf(fmaxf(h2, 0.0f), 2.0f * (float)b.n2 - 1.0f);
+  const uint32_t i0 = min(__float2uint_rz(fmaxf(h0, 0.0f)), 2u * (uint32_t)b.n0 - 1u);
+  const uint32_t i1 = min(__float2uint_rz(fmaxf(h1, 0.0f)), 2u * (uint32_t)b.n1 - 1u);
+  const uint32_t i2 = min(__float2uint_rz(fmaxf(h2, 0.0f)), 2u * (uint32_t)b.n2 - 1u);
   const uint64_t cell = (i0 >> 1) + (uint64_t)b.n0 * ((i1 >> 1) + (uint64_t)b.n1 * (i2 >> 1));
   return (uint32_t)((8 * cell + ((i0 & 1u) | ((i1 & 1u) << 1) | ((i2 & 1u) << 2))) >> b.shift);
 }
