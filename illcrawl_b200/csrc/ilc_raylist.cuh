@@ -125,6 +125,14 @@ __device__ __forceinline__ void locate_axis(float q, float mn, float cs, float h
   sh = min(max(si, 0), 1);
 }
 
+// Rounding of the positions o + z l of a ray up to |z| = zm, and of the cell and
+// subcell found from them: at most a dozen roundings of 2^-24 of the largest term
+// (16 here), in every sum of |o_i| and |zm l_i|.
+__device__ __forceinline__ float ray_rounding(float ox, float oy, float oz, float zm,
+                                              float len_l) {
+  return ((fabsf(ox) + fabsf(oy)) + (fabsf(oz) + zm * len_l)) * 9.5367432e-7f;
+}
+
 // Largest z at which the ray is surely still in [lo, lo + half] along one axis.
 __device__ __forceinline__ float axis_exit(float o, float l, float lo, float half, float margin) {
   if (l > 0.0f) return (lo + half - margin - o) / l;
@@ -284,8 +292,7 @@ __device__ __forceinline__ int build_list(const GridView& g, const char4* __rest
   const char4* order = spiral + sub * 125;
   const float zc = za + 0.5f * (zb - za);
   const float qx = ox + zc * lx, qy = oy + zc * ly, qz = oz + zc * lz;
-  // position rounding: at most a few 2^-24 of the largest term of o + z l
-  const float del = ((fabsf(ox) + fabsf(oy)) + (fabsf(oz) + fabsf(zb) * len_l)) * 9.5367432e-7f;
+  const float del = ray_rounding(ox, oy, oz, fabsf(zb), len_l);
   const float bb = 0.5f * (zb - za) * len_l * 1.00001f + del;
   const float crad = g.cell_radius;
   if (!(bb < 1e15f) || !(crad < 1e15f)) return -1;
@@ -676,16 +683,20 @@ __device__ __forceinline__ void eval_points(const GridView& g, const char4* __re
         if (lead_ok && fabsf(rox) < 1e15f && fabsf(roy) < 1e15f && fabsf(roz) < 1e15f) {
           const float len_l = sqrtf((rlx * rlx + rly * rly) + rlz * rlz);
           float ext = W.meta[lr].ext;
-          // as far as the ray surely stays in the subcell
+          // as far as the ray surely stays in the subcell: the grid's margin
+          // covers the rounding at the grid's own coordinates, the second term
+          // the ray's (a camera thousands of box lengths away)
+          const float zm = fmaxf(fmaxf(fabsf(zlo), fabsf(zhi)), fabsf(zlo + ext));
+          const float keep = g.margin + ray_rounding(rox, roy, roz, zm, len_l);
           const float ex =
               axis_exit(rox, rlx, (g.min0 + (float)bx * g.cs0) + (float)(bs & 1) * g.half0,
-                        g.half0, g.margin);
+                        g.half0, keep);
           const float ey =
               axis_exit(roy, rly, (g.min1 + (float)by * g.cs1) + (float)((bs >> 1) & 1) * g.half1,
-                        g.half1, g.margin);
+                        g.half1, keep);
           const float ez =
               axis_exit(roz, rlz, (g.min2 + (float)bz * g.cs2) + (float)(bs >> 2) * g.half2,
-                        g.half2, g.margin);
+                        g.half2, keep);
           const float reach = fminf(zlo + ext, fminf(ex, fminf(ey, ez)));
           float a = zlo, b = reach > zhi ? reach : zhi;
           int tested = -1;
