@@ -197,10 +197,12 @@ ilc_status build_grid_staged(Context& c, uint64_t n) {
   c.gp = g;
   ILC_CUDA(c, grid_build_device(c, c.tmp_in.as<float4>(), n), "grid build");
   uint32_t flags = 0;
-  ilc_status st = read_flags(c, &flags, nullptr);
+  DevStats ds{};
+  ilc_status st = read_flags(c, &flags, &ds);
   if (st) return st;
   if (flags & FLAG_KEY_RANGE) return fail(c, ILC_ERR_INTERNAL, "particle outside its grid");
   c.n_particles = n;
+  c.even = ds.occupied >= c.gp.total - c.gp.total / 5 && ds.crowded <= n / 1024;
   c.has_grid = true;
   return ILC_OK;
 }
@@ -555,10 +557,12 @@ ilc_status ilc_nn8_setup_particles(ilc_ctx* h, const float* particles, uint64_t 
   c.gp = g;
   ILC_CUDA(c, grid_build_device(c, static_cast<const float4*>(din), n), "grid build");
   uint32_t flags = 0;
-  ilc_status st = read_flags(c, &flags, nullptr);
+  DevStats ds{};
+  ilc_status st = read_flags(c, &flags, &ds);
   if (st) return st;
   if (flags & FLAG_KEY_RANGE) return fail(c, ILC_ERR_INTERNAL, "particle outside its grid");
   c.n_particles = n;
+  c.even = ds.occupied >= c.gp.total - c.gp.total / 5 && ds.crowded <= n / 1024;
   c.has_grid = true;
   // The nn8 lists survive a new particle block: the next query with
   // merge_previous = 1 continues them (reconstructing_data_crawler.cpp:164-255).

@@ -348,22 +348,33 @@ __device__ __forceinline__ uint16_t sub_box_code(const KeyGrid& kg, uint32_t key
 // After the sort, in one pass over the particles: the float4 records in cell
 // order with the sorted->unsorted map (grid3d_sort_particles_into_cells), the
 // cells' [begin, end) over a zeroed cell array (grid3d_determine_cells_begin /
-// _end) and, where codes is not null, the sub-box codes. Bound by the gather's
+// _end) and, where they are not null, the sub-box codes and the counts of occupied
+// cells and of particles in crowded ones. Bound by the gather's
 // 32-byte sectors; three kernels that read the records and the keys again took
 // 25 us for 1,000,003 particles.
 __global__ void finish_kernel(const float4* __restrict__ in, const uint32_t* __restrict__ perm,
                               const uint32_t* __restrict__ sk, uint64_t n, KeyGrid kg,
                               float4* __restrict__ out, uint32_t* __restrict__ s2u,
-                              int2* __restrict__ cells, uint16_t* __restrict__ codes) {
+                              int2* __restrict__ cells, uint16_t* __restrict__ codes,
+                              DevStats* __restrict__ stats) {
   const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const uint32_t j = perm[i], k = sk[i];
-  const float4 p = in[j];
-  if (i == 0 || sk[i - 1] != k) cells[k].x = (int)i;
-  if (i + 1 == n || sk[i + 1] != k) cells[k].y = (int)(i + 1);
-  out[i] = p;
-  s2u[i] = j;
-  if (codes) codes[i] = sub_box_code(kg, k, p);
+  bool first = false, crowd = false;
+  if (i < n) {
+    const uint32_t j = perm[i], k = sk[i];
+    const float4 p = in[j];
+    first = i == 0 || sk[i - 1] != k;
+    if (first) cells[k].x = (int)i;
+    crowd = stats && i >= kCrowd && sk[i - kCrowd] == k;
+    if (i + 1 == n || sk[i + 1] != k) cells[k].y = (int)(i + 1);
+    out[i] = p;
+    s2u[i] = j;
+    if (codes) codes[i] = sub_box_code(kg, k, p);
+  }
+  const int firsts = __syncthreads_count(first), crowded = __syncthreads_count(crowd);
+  if (stats && threadIdx.x == 0) {
+    if (firsts) atomicAdd(&stats->occupied, (unsigned long long)firsts);
+    if (crowded) atomicAdd(&stats->crowded, (unsigned long long)crowded);
+  }
 }
 
 inline unsigned grid_blocks(uint64_t n, int threads) {
@@ -476,7 +487,8 @@ cudaError_t grid_build_device(Context& c, const float4* in, uint64_t n) {
   if ((e = cudaMemsetAsync(c.cells.p, 0, g.total * 8, c.stream))) return e;
   finish_kernel<<<grid_blocks(n, 256), 256, 0, c.stream>>>(
       in, va, ka, n, kg, c.parts.as<float4>(), c.s2u.as<uint32_t>(), c.cells.as<int2>(),
-      c.codes.as<uint16_t>());
+      c.codes.as<uint16_t>(),
+      reinterpret_cast<DevStats*>(c.flags.as<char>() + 64));
   c.launches += 2;  // keys, finish
   return cudaGetLastError();
 }
@@ -636,7 +648,7 @@ extern "C" ilc_status ilc_grid_build_noalloc(const float* particles, uint64_t n,
   if (cudaMemsetAsync(cells, 0, total * 8, st) != cudaSuccess) return ILC_ERR_CUDA;
   finish_kernel<<<grid_blocks(n, 256), 256, 0, st>>>(
       in, va, ka, n, kg, reinterpret_cast<float4*>(sorted_particles), sorted_to_unsorted,
-      reinterpret_cast<int2*>(cells), nullptr);
+      reinterpret_cast<int2*>(cells), nullptr, nullptr);
   uint32_t f = 0;
   if (cudaGetLastError() != cudaSuccess ||
       cudaMemcpyAsync(&f, flags, 4, cudaMemcpyDeviceToHost, st) != cudaSuccess ||

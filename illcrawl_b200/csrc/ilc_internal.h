@@ -61,6 +61,7 @@ struct Context {
   bool has_grid = false;
   uint64_t n_particles = 0;
   GridParams gp{};
+  bool even = false;  // nearly all cells hold particles, hardly any of them many
   DevBuf parts;      // float4 sorted particles
   DevBuf cells;      // int2 per grid cell
   DevBuf s2u;        // uint32 sorted -> original index
@@ -127,9 +128,12 @@ struct DevStats {
   unsigned long long cands;
   unsigned long long max_steps;
   unsigned long long rays_at_limit;
-  unsigned long long pad;
+  unsigned long long occupied;  // grid build: cells with a particle
+  unsigned long long crowded;   // grid build: particles beyond the kCrowd first of their cells
 };
 constexpr size_t kFlagsBytes = 64 + sizeof(DevStats);
+constexpr uint64_t kCrowd = 48;
+constexpr size_t kLeftWord = 8;  // word of the flags: queries left to the warp kernel
 
 // launchers (return cudaError_t of the launch sequence)
 cudaError_t grid_bbox(Context& c, const float4* in, uint64_t n, float* mn3, float* mx3,

@@ -60,7 +60,7 @@ __global__ void query_order_kernel(const uint32_t* __restrict__ first,
   order[first[p.x] + p.y] = (uint32_t)i;
 }
 
-// Slots of one query: squared distances (kMerge: distances, as the lists of the
+// Slots of one query: squared distances (kExact: distances, as the lists of a
 // previous block hold them) and candidate indices.
 struct QuerySlots {
   float d[8];
@@ -69,12 +69,13 @@ struct QuerySlots {
 
 // The walk of nn8_walk() (ilc_device.cuh) for one query; cells whose box lies
 // beyond the search radius are counted and not scanned. Without lists to
-// continue, squared distances stand for distances, as in a list replay
-// (ilc_raylist.cuh). Returns false, with the slots in no defined state, where
-// two of them are too close for that, and at a cell with more than kHard
-// candidates within reach, which one lane would scan while the others wait.
+// continue, squared distances can stand for distances, as in a list replay
+// (ilc_raylist.cuh; kExact: distances themselves). Returns false, with the slots in
+// no defined state, where two of them are too close for that, and at a cell with
+// more than kHard candidates within reach, which one lane would scan while the
+// others wait.
 constexpr int kHard = 96;
-template <bool kMerge>
+template <bool kExact>
 __device__ __forceinline__ bool query_walk(const GridView& g, const char4* __restrict__ spiral,
                                            float qx, float qy, float qz, QuerySlots& s,
                                            WalkStats& st) {
@@ -85,8 +86,8 @@ __device__ __forceinline__ bool query_walk(const GridView& g, const char4* __res
   const char4* order = spiral + (sx + 2 * sy + 4 * sz) * 125;
   const float inf = __int_as_float(0x7f800000);
   float M = max8(s.d);                            // the slot maximum
-  float T = kMerge ? __fmul_ru(M, M) : M;         // squared distances above it cannot enter
-  float rb = (kMerge ? M : fminf(sqrtf(M), FLT_MAX)) + g.cell_radius;
+  float T = kExact ? __fmul_ru(M, M) : M;         // squared distances above it cannot enter
+  float rb = (kExact ? M : fminf(sqrtf(M), FLT_MAX)) + g.cell_radius;
   float rr = rb * rb;
   bool close = false;
 #pragma unroll 1
@@ -122,7 +123,7 @@ __device__ __forceinline__ bool query_walk(const GridView& g, const char4* __res
       const float fx = C.x - qx, fy = C.y - qy, fz = C.z - qz;
       float d = (fx * fx + fy * fy) + fz * fz;
       if (d <= T) {
-        if (kMerge) d = sqrtf(d);
+        if (kExact) d = sqrtf(d);
         if (d < M) {
           bool open = true;  // the first maximal slot
 #pragma unroll
@@ -134,23 +135,23 @@ __device__ __forceinline__ bool query_walk(const GridView& g, const char4* __res
             s.id[q] = hit ? p : s.id[q];
           }
           const float top = max8(s.d);
-          if (!kMerge) close = close || (M < inf && top >= M * 0.99999952f);
+          if (!kExact) close = close || (M < inf && top >= M * 0.99999952f);
           M = top;
-          T = kMerge ? __fmul_ru(M, M) : M;
+          T = kExact ? __fmul_ru(M, M) : M;
         }
       }
     }
     if (M != before) {
-      rb = (kMerge ? M : fminf(sqrtf(M), FLT_MAX)) + g.cell_radius;
+      rb = (kExact ? M : fminf(sqrtf(M), FLT_MAX)) + g.cell_radius;
       rr = rb * rb;
     }
   }
   return !close;
 }
 
-// One query per lane, in bin order; those that query_walk() gives up are listed
-// in hard[0..].
-template <bool kMerge>
+// One query per lane, in the given order or that of their bins; those that
+// query_walk() gives up are listed in hard[0..]. kMerge implies kExact.
+template <bool kMerge, bool kExact>
 __global__ void __launch_bounds__(256)
 nn8_query_kernel(const __grid_constant__ GridView g, const char4* __restrict__ spiral_g,
                  const float4* __restrict__ pts, const uint32_t* __restrict__ order, uint64_t n,
@@ -170,11 +171,11 @@ nn8_query_kernel(const __grid_constant__ GridView g, const char4* __restrict__ s
     for (int j = 0; j < 8; ++j) {
       // Lists carry original indices; entries kept from the previous call are
       // tagged with the top bit so they are not mapped through this grid's s2u.
-      s.d[j] = kMerge ? list_d[8 * i + j] : __int_as_float(0x7f800000);
+      s.d[j] = kMerge ? list_d[8 * i + j] : kExact ? FLT_MAX : __int_as_float(0x7f800000);
       const int32_t o = kMerge ? list_id[8 * i + j] : -1;
       s.id[j] = o >= 0 ? (int32_t)(0x80000000u | (uint32_t)o) : -1;
     }
-    if (!query_walk<kMerge>(g, spiral, q.x, q.y, q.z, s, st)) {
+    if (!query_walk<kExact>(g, spiral, q.x, q.y, q.z, s, st)) {
       st.cells = st.cands = 0;
       hard[atomicAdd(n_hard, 1u)] = (uint32_t)i;
     } else {
@@ -184,7 +185,7 @@ nn8_query_kernel(const __grid_constant__ GridView g, const char4* __restrict__ s
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         const int32_t id = s.id[j];
-        if (!kMerge) s.d[j] = id < 0 ? FLT_MAX : sqrtf(s.d[j]);
+        if (!kExact) s.d[j] = id < 0 ? FLT_MAX : sqrtf(s.d[j]);
         v[j] = id >= 0 ? __ldg(&g.parts[id].w) : (kMerge ? list_v[8 * i + j] : 0.0f);
         w[j] = weight3d(s.d[j]);
       }
@@ -581,24 +582,21 @@ nn8_query_warp_kernel(const __grid_constant__ GridView g, const char4* __restric
 GridView make_grid_view(const Context& c);
 
 // The queries ordered by bin (a counting sort; the order within a bin is the
-// atomics', which no result depends on).
-cudaError_t query_order(Context& c, const GridView& g, const float4* pts, uint64_t n,
-                        const uint32_t** order, uint32_t** left) {
+// atomics', which no result depends on). `at`: words of query_sort in front.
+cudaError_t query_order(Context& c, const GridView& g, const float4* pts, uint64_t n, size_t at,
+                        const uint32_t** order) {
   cudaError_t e;
   QueryBins b{g.n0, g.n1, g.n2, 0};
   while (((8 * c.gp.total - 1) >> b.shift) >= (1ull << kBinBits)) ++b.shift;
   const uint64_t bins = ((8 * c.gp.total - 1) >> b.shift) + 1;
-  // counts (then first positions), scan scratch, counter and list of the
-  // queries left to the warp kernel, places, order
-  const uint64_t scan_words = scan_scratch_words(bins);
-  const size_t words = (bins + 3) / 4 * 4, off_left = words + (scan_words + 3) / 4 * 4,
-               off_place = off_left + 4 + (n + 3) / 4 * 4;
-  if ((e = c.query_sort.ensure((off_place + 3 * n) * 4))) return e;
-  uint32_t* count = c.query_sort.as<uint32_t>();
+  // counts (then first positions), scan scratch, places, order
+  const size_t words = (bins + 3) / 4 * 4,
+               off_place = words + (scan_scratch_words(bins) + 3) / 4 * 4;
+  if ((e = c.query_sort.ensure((at + off_place + 3 * n) * 4))) return e;
+  uint32_t* count = c.query_sort.as<uint32_t>() + at;
   uint2* place = reinterpret_cast<uint2*>(count + off_place);
   uint32_t* ord = reinterpret_cast<uint32_t*>(place + n);
-  *left = count + off_left;
-  if ((e = cudaMemsetAsync(count, 0, (off_left + 4) * 4, c.stream))) return e;
+  if ((e = cudaMemsetAsync(count, 0, off_place * 4, c.stream))) return e;
   const unsigned blocks = (unsigned)((n + 255) / 256);
   query_count_kernel<<<blocks, 256, 0, c.stream>>>(g, b, pts, n, count, place);
   c.launches += 2;
@@ -608,12 +606,25 @@ cudaError_t query_order(Context& c, const GridView& g, const float4* pts, uint64
   return cudaGetLastError();
 }
 
-// Queries from which on ILC_QUERY_THREAD walks one query per lane. Fewer leave
-// SMs idle that way, and the slowest lane's chain of loads (150-250 us) is the
-// time: warp and lane walks take 34 / 175 us for 1,000 queries, 184 / 165-247 us
-// for 65,537, 331 / 180-280 us for 131,072 and 2,360 / 510-860 us for 1,048,576
-// (20,000 to 4,194,304 particles).
+// Queries from which on ILC_QUERY_THREAD walks one query per lane, and from
+// which on it orders them first. Fewer leave SMs idle that way, and the slowest
+// lane's chain of loads (150-250 us among clustered particles) is the time: warp
+// and ordered lane walks take 34 / 175 us for 1,000 queries, 184 / 165-247 us for
+// 65,537, 331 / 180-280 us for 131,072 and 2,360 / 510-860 us for 1,048,576
+// (20,000 to 4,194,304 particles of a halo, whose grids have 3-30 % of their cells
+// occupied).
 constexpr uint64_t kThreadMin = 81920;
+// In an even grid (Context::even: particles in four of five cells or more, at most
+// a thousandth of them beyond the 48th of their cell) no lane's walk is long and
+// order gains little: from 40,960 queries on the lanes are ahead of the warps, and
+// up to 393,216 the sort costs more than it saves. A few queries whose distances are
+// too close for squared ones would cost the warp kernel's latency (65,537 random
+// queries in 116 us, 81,000 in 135), so such grids are walked on rounded distances.
+// Whole calls in us, 100,000 uniform particles, random queries (in the order of their
+// cells): 65,537 by warps 165 (158), ordered lanes 135 (131), lanes 101 (86); 81,000:
+// 198 (192), 147 (142), 109 (92); 200,000: 439 (418), 189 (183), 168 (130); 394,000
+// ordered 235 (228), 393,000 unordered 246 (196).
+constexpr uint64_t kEvenMin = 40960, kEvenOrder = 393216;
 
 cudaError_t nn8_query_launch(Context& c, const float4* pts, uint64_t n, bool merge, float* out,
                              int32_t* idx8, float* d8) {
@@ -627,19 +638,26 @@ cudaError_t nn8_query_launch(Context& c, const float4* pts, uint64_t n, bool mer
   unsigned long long* stats =
       reinterpret_cast<unsigned long long*>(c.flags.as<char>() + 64);
   const uint32_t *hard = nullptr, *n_hard = nullptr;
-  if (c.query_engine == ILC_QUERY_THREAD && n >= kThreadMin && n <= 0xffffffffull) {
+  const bool even = c.even;
+  if (c.query_engine == ILC_QUERY_THREAD && n >= (even ? kEvenMin : kThreadMin) &&
+      n <= 0xffffffffull) {
+    // the list of the queries left to the warp kernel, then the sort's arrays
     const uint32_t* order = nullptr;
-    uint32_t* left = nullptr;
-    if ((e = query_order(c, g, pts, n, &order, &left))) return e;
+    const size_t list = (n + 3) / 4 * 4;
+    if ((e = even && n < kEvenOrder ? c.query_sort.ensure(list * 4)
+                                    : query_order(c, g, pts, n, list, &order)))
+      return e;
+    uint32_t* left = c.query_sort.as<uint32_t>();
+    uint32_t* n_left = c.flags.as<uint32_t>() + kLeftWord;
     ++c.launches;
-    const auto kernel = merge ? nn8_query_kernel<true> : nn8_query_kernel<false>;
+    const auto kernel = merge ? nn8_query_kernel<true, true> : even ? nn8_query_kernel<false, true> : nn8_query_kernel<false, false>;
     kernel<<<(unsigned)((n + 255) / 256), 256, 0, c.stream>>>(
-        g, c.spiral.as<char4>(), pts, order, n, left + 4, left, c.list_d.as<float>(),
+        g, c.spiral.as<char4>(), pts, order, n, left, n_left, c.list_d.as<float>(),
         c.list_v.as<float>(), c.list_id.as<int32_t>(), out, idx8, d8, c.s2u.as<uint32_t>(),
         stats);
     if ((e = cudaGetLastError())) return e;
-    n_hard = left;
-    hard = left + 4;
+    n_hard = n_left;
+    hard = left;
   }
   // one warp per query; persistent blocks of 8 warps, as many as are resident
   int sms = 0, per_sm = 0;
