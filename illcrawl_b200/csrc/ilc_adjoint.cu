@@ -18,6 +18,7 @@
 #include "ilc_internal.h"
 #include "ilc_quantity.cuh"
 #include "ilc_raylist.cuh"
+#include "ilc_walk4.cuh"
 
 namespace ilc {
 
@@ -206,7 +207,17 @@ struct AdjK {
   unsigned long long n_rays;       // 128 per 16 x 8 tile
   unsigned tiles_x;
   float4* over;                    // list overflow, kOver per resident ray
+  LeaveRule leave;                 // a forward pass that walked first: the rays it left
 };
+
+// Pixel of ray q, numbered as in the render kernel.
+__device__ __forceinline__ void adjoint_pixel(const AdjK& a, unsigned long long q, int& ix,
+                                              int& iy) {
+  const unsigned tile = (unsigned)(q >> 7), t = (unsigned)(q & 127u);
+  const int sub = (int)(t >> 3);
+  ix = (int)(tile % a.tiles_x) * 16 + (sub & 3) * 4 + (int)(t & 3u);
+  iy = a.row0 + (int)(tile / a.tiles_x) * 8 + (sub >> 2) * 2 + (int)((t >> 2) & 1u);
+}
 
 constexpr int kAdjBlocks = 4;
 
@@ -253,13 +264,10 @@ adjoint_kernel(const __grid_constant__ AdjK a, const __grid_constant__ GridView 
       const unsigned long long q = take_rays(a.queue, want, fresh, lane, wg);
       fresh = false;
       if (!have && !drained) {
-        drained = q >= a.n_rays;
+        drained = q >= list_rays(a.leave, a.n_rays);
         if (!drained) {
-          const unsigned tile = (unsigned)(q >> 7), t = (unsigned)(q & 127u);
-          const int sub = (int)(t >> 3);
-          const int ix = (int)(tile % a.tiles_x) * 16 + (sub & 3) * 4 + (int)(t & 3u);
-          const int iy =
-              a.row0 + (int)(tile / a.tiles_x) * 8 + (sub >> 2) * 2 + (int)((t >> 2) & 1u);
+          int ix, iy;
+          adjoint_pixel(a, list_ray(a.leave, q), ix, iy);
           if (ix < a.cam.nx && iy < a.row_end) {
             gi = a.seed[(int64_t)iy * a.cam.nx + ix];
             have = gi != 0.0f;
@@ -332,6 +340,90 @@ adjoint_kernel(const __grid_constant__ AdjK a, const __grid_constant__ GridView 
   }
   atomicAdd(&stats[3], (unsigned long long)ws.cells);
   atomicAdd(&stats[4], (unsigned long long)ws.cands);
+}
+
+// Point J's slots of a walked step as the scatter needs them.
+template <int J> __device__ __forceinline__ void scatter_slots(const Step4& s, ScatterSlots& o) {
+  s4_weights<J>(s, o.w, o.ws);
+#pragma unroll
+  for (int t = 0; t < 8; ++t) o.id[t] = __float_as_int(s4_v(s, J, t));
+}
+template <int J>
+__device__ __forceinline__ void scatter_point(const Step4& s, float c, double* __restrict__ grad) {
+  ScatterSlots o;
+  scatter_slots<J>(s, o);
+  scatter(o, (double)c, grad);
+}
+
+// The rays that a forward pass walked to their end, a ray per thread, as it walked
+// them (walk_kernel in ilc_render.cu): their steps are long against a cell.
+__global__ void __launch_bounds__(kSlotThreads, kAdjBlocks)
+adjoint_walk_kernel(const __grid_constant__ AdjK a, const __grid_constant__ GridView g,
+                    const char4* __restrict__ spiral_g, uint32_t* __restrict__ flags,
+                    unsigned long long* __restrict__ stats) {
+  __shared__ char4 spiral[1000];
+  __shared__ SlotMem slot_mem;
+  __shared__ unsigned long long next_tile;
+  load_spiral(spiral, spiral_g);
+  const float lx = a.cam.look0, ly = a.cam.look1, lz = a.cam.look2;
+  const float fa = (float)a.atol, fr = (float)a.rtol;
+  const bool replay = a.mode == ILC_ADJOINT_CHECKPOINT;
+  for (;;) {
+    if (threadIdx.x == 0) next_tile = atomicAdd(a.queue + 1, 1ull);
+    __syncthreads();
+    const unsigned long long q = 128 * next_tile + walk_ray();
+    __syncthreads();
+    if (q >= a.n_rays) break;  // (all of the block)
+    if ((a.leave.left[q >> 3] >> (q & 7u)) & 1u) continue;
+    int ix, iy;
+    adjoint_pixel(a, q, ix, iy);
+    if (ix >= a.cam.nx || iy >= a.row_end) continue;
+    const float gi = a.seed[(int64_t)iy * a.cam.nx + ix];
+    if (gi == 0.0f) continue;
+    const int64_t ray = (int64_t)(iy - a.row0) * a.cam.nx + ix;  // in the launch's rows
+    float px, py, pz;
+    pixel_corner(a.cam, ix, iy, px, py, pz);
+    const int64_t limit = replay ? a.rec_n[ray] : a.max_steps;
+    const float* hs = replay ? a.rec_h + ray * a.rec_cap : nullptr;
+    float I = 0.0f, z = a.z0, h = 1.0f, k1 = 0.0f;
+    unsigned long long steps = 0;
+    ScatterSlots prev;  // point 2 of the last accepted step: the next one's k1
+    double prev_c = 0.0;
+    bool have_prev = false;
+    WalkStats ws;
+    while ((int64_t)steps < limit && (replay || z < a.z_end)) {
+      if (replay) h = hs[steps];
+      float pts[4];
+      rkf_points(z, h, pts);
+      Step4 s;
+      s4_bind(s, slot_mem);
+      nn8_walk_step4<true>(g, spiral, px, py, pz, lx, ly, lz, pts, s, ws);
+      const float zb = z, hb = h;
+      if (replay) {
+        z += h;
+      } else {
+        const float e[4] = {s4_value<0, true>(g, s), s4_value<1, true>(g, s),
+                            s4_value<2, true>(g, s), s4_value<3, true>(g, s)};
+        if (a.controller == ILC_CONTROLLER_REF32)
+          rkf_advance_ref32(I, z, h, k1, fa, fr, a.z_end, e, kEps, kHmin, kHmax, pts);
+        else
+          rkf_advance_fp64(I, z, h, k1, a.atol, a.rtol, a.z_end, e, kEps, kHmin, kHmax, pts);
+      }
+      ++steps;
+      if (!replay && z == zb) continue;
+      scatter_point<0>(s, gi * (hb * 1408.f / 2565.f), a.grad);
+      scatter_point<1>(s, gi * (hb * 2197.f / 4101.f), a.grad);
+      if (have_prev) scatter(prev, prev_c + (double)(gi * (hb * 25.f / 216.f)), a.grad);
+      scatter_slots<2>(s, prev);
+      prev_c = (double)(gi * (-hb / 5.f));
+      have_prev = true;
+    }
+    if (have_prev) scatter(prev, prev_c, a.grad);
+    if (!replay && z < a.z_end) atomicOr(flags, FLAG_STEP_LIMIT);
+    atomicAdd(&stats[0], steps);
+    atomicAdd(&stats[3], (unsigned long long)ws.cells);
+    atomicAdd(&stats[4], (unsigned long long)ws.cands);
+  }
 }
 
 // dL/dln rho and dL/dln T in the original particle order.
@@ -407,14 +499,18 @@ cudaError_t adjoint_ray_launch(Context& c, const RenderArgs& r, int mode, const 
       (unsigned long long)k.tiles_x * (unsigned)((k.row_end - k.row0 + 7) / 8);
   k.n_rays = 128ull * tiles;
   if ((e = c.tile_queue.ensure(256))) return e;
-  if ((e = cudaMemsetAsync(c.tile_queue.p, 0, 8, c.stream))) return e;
+  if ((e = cudaMemsetAsync(c.tile_queue.p, 0, 16, c.stream))) return e;
   k.queue = c.tile_queue.as<unsigned long long>();
-  int sms = 0, per_sm = 0;
+  // (the rays of the forward pass over the same rows)
+  k.leave = c.leave;
+  int sms = 0, per_sm = 0, per_sm_w = 0;
   if ((e = cudaFuncSetAttribute(adjoint_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)sizeof(AdjMem))) ||
       (e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c.device)) ||
       (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, adjoint_kernel, kListThreads,
-                                                         sizeof(AdjMem))))
+                                                         sizeof(AdjMem))) ||
+      (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_w, adjoint_walk_kernel,
+                                                         kSlotThreads, 0)))
     return e;
   const unsigned long long resident = (unsigned long long)sms * (per_sm > 0 ? per_sm : 1);
   // (down to one ray per warp)
@@ -426,6 +522,14 @@ cudaError_t adjoint_ray_launch(Context& c, const RenderArgs& r, int mode, const 
     if ((e = cudaEventCreate(&c.ev0)) || (e = cudaEventCreate(&c.ev1))) return e;
   }
   cudaEventRecord(c.ev0, c.stream);
+  if (k.leave.left) {
+    const unsigned long long fit = (unsigned long long)sms * (per_sm_w > 0 ? per_sm_w : 1);
+    ++c.launches;
+    adjoint_walk_kernel<<<(unsigned)(fit < tiles ? fit : tiles), kSlotThreads, 0, c.stream>>>(
+        k, g, c.spiral.as<char4>(), c.flags.as<uint32_t>(),
+        reinterpret_cast<unsigned long long*>(c.flags.as<char>() + 64));
+    if ((e = cudaGetLastError())) return e;
+  }
   ++c.launches;
   adjoint_kernel<<<blocks, kListThreads, sizeof(AdjMem), c.stream>>>(
       k, g, c.spiral.as<char4>(), c.flags.as<uint32_t>(),

@@ -25,6 +25,7 @@
 #include "ilc_device.cuh"
 #include "ilc_internal.h"
 #include "ilc_raylist.cuh"
+#include "ilc_walk4.cuh"
 
 namespace ilc {
 
@@ -46,7 +47,27 @@ struct BatchK {
   const uint32_t* order;
   unsigned long long* queue;
   float4* over;   // list overflow, kOver per resident ray
+  LeaveRule leave;  // rays walked first, and those left to the lists
+  float* walk_state;  // state of the walk kernel's rays, 4 V floats per thread
 };
+
+// Ray ti of work item `item`: its job and pixel; false outside the image.
+__device__ __forceinline__ bool item_pixel(const BatchK& a, const JobDev& J, uint64_t item, int ti,
+                                           int& ix, int& iy) {
+  const uint64_t t = item - J.item_begin;
+  if (a.tile_w > 0) {  // compact tile of tile_w x (32 / tile_w) pixels
+    const int tx = (int)(t % (uint64_t)J.tiles_x), ty = (int)(t / (uint64_t)J.tiles_x);
+    ix = tx * a.tile_w + ti % a.tile_w;
+    iy = ty * (32 / a.tile_w) + ti / a.tile_w;
+    return ix < J.nx && iy < J.ny;
+  }
+  // strided: pixels t, t + T, t + 2T, ... (T = items of the job)
+  const uint64_t pix = t + (uint64_t)ti * (uint64_t)J.tiles_x;
+  const bool inside = pix < (uint64_t)J.nx * (uint64_t)J.ny;
+  ix = inside ? (int)(pix % (uint64_t)J.nx) : J.nx;
+  iy = inside ? (int)(pix / (uint64_t)J.nx) : J.ny;
+  return inside;
+}
 
 // Largest k with jobs[k].item_begin <= item.
 __device__ __forceinline__ int find_job(const JobDev* __restrict__ jobs, int n, uint64_t item) {
@@ -135,6 +156,136 @@ struct ChanHand {
   float ws[4][kRays];   // sum of point j's weights
 };
 
+struct ListHand {
+  const ChanHand& h;
+  int r;
+  __device__ __forceinline__ float w(int p, int q) const { return h.w[p * 8 + q][r]; }
+  __device__ __forceinline__ int id(int p, int q) const { return h.id[p * 8 + q][r]; }
+  __device__ __forceinline__ float ws(int p) const { return h.ws[p][r]; }
+};
+
+// The step (zr, hr) of one ray for all channels, by a whole warp: the channels'
+// values at the 4 points (from the slots' weights and indices in H), the joint step
+// control, and the ray's state (I[V], k1[V] and room for their candidates) if the
+// step is accepted. nh: the next step size.
+template <class Hand>
+__device__ __forceinline__ bool channels_step(const BatchK& a, const Hand& H, float* Is, float zr,
+                                              float hr, int lane, double& nh) {
+  float* Ks = Is + a.V;
+  const double hd = (double)hr;
+  const double zd = (double)(zr + hr), rz = 1.0 / zd;
+  double xl = __longlong_as_double(0x7ff0000000000000ll);  // +inf
+  bool x0nan = false;
+  // candidate values (I + delta4, k5): a lane's last group stays in
+  // registers, earlier ones (V > 128) go to the ray's scratch half; they
+  // are committed once the warp knows the step is accepted
+  float* Es = Ks + a.V;
+  float* E2s = Es + a.V;
+  int held = -1;
+  float4 hi4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f), hk4 = hi4;
+  if ((a.V & 3) == 0) {
+    // rows of V = 4G floats: lane handles float4 groups lane, lane+32, ...
+    // (channels 4g..4g+3), one 16-byte load per neighbour and group
+    const int G = a.V >> 2;
+    const float4* __restrict__ chan4 = reinterpret_cast<const float4*>(a.chan);
+#pragma unroll 1
+    for (int gi = lane; gi < G; gi += 32) {
+      if (held >= 0) {
+        reinterpret_cast<float4*>(Es)[held] = hi4;
+        reinterpret_cast<float4*>(E2s)[held] = hk4;
+      }
+      held = gi;
+      const float4 i4 = reinterpret_cast<const float4*>(Is)[gi];
+      const float4 k4 = reinterpret_cast<const float4*>(Ks)[gi];
+      float ev[4][4];
+#pragma unroll
+      for (int p = 0; p < 4; ++p) {
+        float dot[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          const int id = H.id(p, q);
+          const float4 v = id >= 0 ? __ldg(&chan4[(size_t)id * G + gi])
+                                   : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+          const float wq = H.w(p, q);
+          dot[0] = __fmaf_rn(wq, v.x, dot[0]);
+          dot[1] = __fmaf_rn(wq, v.y, dot[1]);
+          dot[2] = __fmaf_rn(wq, v.z, dot[2]);
+          dot[3] = __fmaf_rn(wq, v.w, dot[3]);
+        }
+        const float wsum = H.ws(p);
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          ev[p][k] = (wsum != 0.0f && dot[k] != 0.0f) ? dot[k] / wsum : 0.0f;
+      }
+      const float ic[4] = {i4.x, i4.y, i4.z, i4.w}, kc[4] = {k4.x, k4.y, k4.z, k4.w};
+      float en[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        double x;
+        en[k] = channel_step(ic[k], kc[k], ev[0][k], ev[1][k], ev[2][k], ev[3][k], hd, zd,
+                             rz, a.atol, a.rtol, x);
+        if (gi == 0 && k == 0 && isnan(x)) x0nan = true;
+        xl = fmin(xl, x);
+      }
+      hi4 = make_float4(en[0], en[1], en[2], en[3]);
+      hk4 = make_float4(ev[2][0], ev[2][1], ev[2][2], ev[2][3]);
+    }
+  } else {
+#pragma unroll 1
+    for (int c = lane; c < a.V; c += 32) {
+      float ev[4];
+#pragma unroll
+      for (int p = 0; p < 4; ++p) {
+        float dot = 0.0f;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          const int id = H.id(p, q);
+          const float v = id >= 0 ? __ldg(&a.chan[(size_t)id * a.V + c]) : 0.0f;
+          dot = __fmaf_rn(H.w(p, q), v, dot);
+        }
+        const float wsum = H.ws(p);
+        ev[p] = (wsum != 0.0f && dot != 0.0f) ? dot / wsum : 0.0f;
+      }
+      double x;
+      Es[c] = channel_step(Is[c], Ks[c], ev[0], ev[1], ev[2], ev[3], hd, zd, rz, a.atol,
+                           a.rtol, x);
+      E2s[c] = ev[2];
+      if (c == 0 && isnan(x)) x0nan = true;
+      xl = fmin(xl, x);
+    }
+  }
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) xl = fmin(xl, __shfl_xor_sync(kAll, xl, off));
+  // The host-side definition takes x_0 and then every smaller x_c:
+  // a NaN x_0 gives NaN, any other NaN is passed over.
+  const bool n0 = __shfl_sync(kAll, x0nan, 0);
+  const double xmin = n0 ? __longlong_as_double(0x7ff8000000000000ll) : xl;
+  double sc = sqrt(sqrt(xmin));
+  nh = sc * hd;
+  if (nh < (double)kHmin) nh = (double)kHmin;
+  else if (nh > (double)kHmax) nh = (double)kHmax;
+  sc = nh / hd;
+  const bool accept = !(sc < 0.95);
+  if (accept) {
+    if (held >= 0) {
+      reinterpret_cast<float4*>(Is)[held] = hi4;
+      reinterpret_cast<float4*>(Ks)[held] = hk4;
+#pragma unroll 1
+      for (int gi = lane; gi < held; gi += 32) {
+        reinterpret_cast<float4*>(Is)[gi] = reinterpret_cast<const float4*>(Es)[gi];
+        reinterpret_cast<float4*>(Ks)[gi] = reinterpret_cast<const float4*>(E2s)[gi];
+      }
+    } else if ((a.V & 3) != 0) {
+#pragma unroll 1
+      for (int c = lane; c < a.V; c += 32) {
+        Is[c] = Es[c];
+        Ks[c] = E2s[c];
+      }
+    }
+  }
+  return accept;
+}
+
 template <bool kMulti> struct BlockMem {
   char4 spiral[1000];
   WarpLists lists[kListWarps];
@@ -143,6 +294,8 @@ template <bool kMulti> struct BlockMem {
   // steps of a ray, rays at the step limit)
   unsigned long long stats[7];
 };
+
+constexpr int kWalkBlocks = 4;  // per SM
 
 // kMulti: V > 1 channels from the table; the slots carry sorted indices.
 // Otherwise they carry the values (V = 1: the table's, or the particles' own
@@ -165,12 +318,10 @@ batched_kernel(const __grid_constant__ BatchK a, const __grid_constant__ GridVie
   const unsigned wg = blockIdx.x * kListWarps + warp;
   if (lane == 0) W.over = a.over + (size_t)wg * kRays * kOver;
   ChanHand& H = M.hand[kMulti ? warp : 0];
-  const int tw = a.tile_w, th = a.tile_w > 0 ? 32 / a.tile_w : 1;
   float* wstate = kMulti ? a.state + ((size_t)blockIdx.x * kListThreads / 4 +
                                       (size_t)warp * kRays) * 4 * (size_t)a.V
                          : nullptr;
   const float ext0 = 0.06f * g.cs0;
-  const unsigned long long n_rays = 32ull * a.n_items;
   // this group's ray
   bool have = false, drained = false, fresh = true;
   float ox = 0.0f, oy = 0.0f, oz = 0.0f, lx = 0.0f, ly = 0.0f, lz = 0.0f, len = 0.0f;
@@ -186,27 +337,15 @@ batched_kernel(const __grid_constant__ BatchK a, const __grid_constant__ GridVie
       const unsigned long long q = take_rays(a.queue, want, fresh, lane, wg);
       fresh = false;
       if (!have && !drained) {
-        if (q >= n_rays) {
+        if (q >= list_rays(a.leave, 32ull * a.n_items)) {
           drained = true;
         } else {
-          const unsigned long long qi = q >> 5;
-          const int ti = (int)(q & 31);
+          const unsigned long long ray = list_ray(a.leave, q);
+          const unsigned long long qi = ray >> 5;
           const uint64_t item = a.order ? (uint64_t)a.order[qi] : qi;
           const JobDev& J = a.jobs[find_job(a.jobs, a.n_jobs, item)];
-          const uint64_t t = item - J.item_begin;
           int ix, iy;
-          bool inside;
-          if (tw > 0) {  // compact tile of tw x th pixels
-            const int tx = (int)(t % (uint64_t)J.tiles_x), ty = (int)(t / (uint64_t)J.tiles_x);
-            ix = tx * tw + ti % tw;
-            iy = ty * th + ti / tw;
-            inside = ix < J.nx && iy < J.ny;
-          } else {       // strided: pixels t, t + T, t + 2T, ... (T = items of the job)
-            const uint64_t pix = t + (uint64_t)ti * (uint64_t)J.tiles_x;
-            inside = pix < (uint64_t)J.nx * (uint64_t)J.ny;
-            ix = inside ? (int)(pix % (uint64_t)J.nx) : J.nx;
-            iy = inside ? (int)(pix / (uint64_t)J.nx) : J.ny;
-          }
+          const bool inside = item_pixel(a, J, item, (int)(ray & 31), ix, iy);
           if (inside) {
             bool masked;
             float o[3];
@@ -280,119 +419,9 @@ batched_kernel(const __grid_constant__ BatchK a, const __grid_constant__ GridVie
         const int gl = __ffs(gom) - 1, tr = gl >> 2;
         gom &= gom - 1;
         const float zr = __shfl_sync(kAll, z, gl), hr = __shfl_sync(kAll, h, gl);
-        float* Is = wstate + (size_t)tr * 4 * a.V;
-        float* Ks = Is + a.V;
-        const double hd = (double)hr;
-        const double zd = (double)(zr + hr), rz = 1.0 / zd;
-        double xl = __longlong_as_double(0x7ff0000000000000ll);  // +inf
-        bool x0nan = false;
-        // candidate values (I + delta4, k5): a lane's last group stays in
-        // registers, earlier ones (V > 128) go to the ray's scratch half; they
-        // are committed once the warp knows the step is accepted
-        float* Es = Ks + a.V;
-        float* E2s = Es + a.V;
-        int held = -1;
-        float4 hi4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f), hk4 = hi4;
-        if ((a.V & 3) == 0) {
-          // rows of V = 4G floats: lane handles float4 groups lane, lane+32, ...
-          // (channels 4g..4g+3), one 16-byte load per neighbour and group
-          const int G = a.V >> 2;
-          const float4* __restrict__ chan4 = reinterpret_cast<const float4*>(a.chan);
-#pragma unroll 1
-          for (int gi = lane; gi < G; gi += 32) {
-            if (held >= 0) {
-              reinterpret_cast<float4*>(Es)[held] = hi4;
-              reinterpret_cast<float4*>(E2s)[held] = hk4;
-            }
-            held = gi;
-            const float4 i4 = reinterpret_cast<const float4*>(Is)[gi];
-            const float4 k4 = reinterpret_cast<const float4*>(Ks)[gi];
-            float ev[4][4];
-#pragma unroll
-            for (int p = 0; p < 4; ++p) {
-              float dot[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll
-              for (int q = 0; q < 8; ++q) {
-                const int id = H.id[p * 8 + q][tr];
-                const float4 v = id >= 0 ? __ldg(&chan4[(size_t)id * G + gi])
-                                         : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                const float wq = H.w[p * 8 + q][tr];
-                dot[0] = __fmaf_rn(wq, v.x, dot[0]);
-                dot[1] = __fmaf_rn(wq, v.y, dot[1]);
-                dot[2] = __fmaf_rn(wq, v.z, dot[2]);
-                dot[3] = __fmaf_rn(wq, v.w, dot[3]);
-              }
-              const float wsum = H.ws[p][tr];
-#pragma unroll
-              for (int k = 0; k < 4; ++k)
-                ev[p][k] = (wsum != 0.0f && dot[k] != 0.0f) ? dot[k] / wsum : 0.0f;
-            }
-            const float ic[4] = {i4.x, i4.y, i4.z, i4.w}, kc[4] = {k4.x, k4.y, k4.z, k4.w};
-            float en[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              double x;
-              en[k] = channel_step(ic[k], kc[k], ev[0][k], ev[1][k], ev[2][k], ev[3][k], hd, zd,
-                                   rz, a.atol, a.rtol, x);
-              if (gi == 0 && k == 0 && isnan(x)) x0nan = true;
-              xl = fmin(xl, x);
-            }
-            hi4 = make_float4(en[0], en[1], en[2], en[3]);
-            hk4 = make_float4(ev[2][0], ev[2][1], ev[2][2], ev[2][3]);
-          }
-        } else {
-#pragma unroll 1
-          for (int c = lane; c < a.V; c += 32) {
-            float ev[4];
-#pragma unroll
-            for (int p = 0; p < 4; ++p) {
-              float dot = 0.0f;
-#pragma unroll
-              for (int q = 0; q < 8; ++q) {
-                const int id = H.id[p * 8 + q][tr];
-                const float v = id >= 0 ? __ldg(&a.chan[(size_t)id * a.V + c]) : 0.0f;
-                dot = __fmaf_rn(H.w[p * 8 + q][tr], v, dot);
-              }
-              const float wsum = H.ws[p][tr];
-              ev[p] = (wsum != 0.0f && dot != 0.0f) ? dot / wsum : 0.0f;
-            }
-            double x;
-            Es[c] = channel_step(Is[c], Ks[c], ev[0], ev[1], ev[2], ev[3], hd, zd, rz, a.atol,
-                                 a.rtol, x);
-            E2s[c] = ev[2];
-            if (c == 0 && isnan(x)) x0nan = true;
-            xl = fmin(xl, x);
-          }
-        }
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) xl = fmin(xl, __shfl_xor_sync(kAll, xl, off));
-        // The host-side definition takes x_0 and then every smaller x_c:
-        // a NaN x_0 gives NaN, any other NaN is passed over.
-        const bool n0 = __shfl_sync(kAll, x0nan, 0);
-        const double xmin = n0 ? __longlong_as_double(0x7ff8000000000000ll) : xl;
-        double sc = sqrt(sqrt(xmin));
-        double nh = sc * hd;
-        if (nh < (double)kHmin) nh = (double)kHmin;
-        else if (nh > (double)kHmax) nh = (double)kHmax;
-        sc = nh / hd;
-        const bool accept = !(sc < 0.95);
-        if (accept) {
-          if (held >= 0) {
-            reinterpret_cast<float4*>(Is)[held] = hi4;
-            reinterpret_cast<float4*>(Ks)[held] = hk4;
-#pragma unroll 1
-            for (int gi = lane; gi < held; gi += 32) {
-              reinterpret_cast<float4*>(Is)[gi] = reinterpret_cast<const float4*>(Es)[gi];
-              reinterpret_cast<float4*>(Ks)[gi] = reinterpret_cast<const float4*>(E2s)[gi];
-            }
-          } else if ((a.V & 3) != 0) {
-#pragma unroll 1
-            for (int c = lane; c < a.V; c += 32) {
-              Is[c] = Es[c];
-              Ks[c] = E2s[c];
-            }
-          }
-        }
+        double nh;
+        const bool accept = channels_step(
+            a, ListHand{H, tr}, wstate + (size_t)tr * 4 * a.V, zr, hr, lane, nh);
         if (r == tr) {
           my_acc = accept;
           my_nh = nh;
@@ -440,6 +469,169 @@ batched_kernel(const __grid_constant__ BatchK a, const __grid_constant__ GridVie
     atomicAdd(&stats[4], M.stats[4]);
     atomicMax(&stats[5], M.stats[5]);
     atomicAdd(&stats[6], M.stats[6]);
+  }
+}
+
+// V > 1, a walked ray: weights in the distance rows of its slot columns, indices in
+// the value rows.
+struct WalkHand {
+  const SlotMem& m;
+  const float (*sum)[kSlotThreads];
+  int t;
+  __device__ __forceinline__ float w(int p, int q) const { return m.d[p * 8 + q][t]; }
+  __device__ __forceinline__ int id(int p, int q) const {
+    return __float_as_int(m.v[p * 8 + q][t]);
+  }
+  __device__ __forceinline__ float ws(int p) const { return sum[p][t]; }
+};
+
+// Point J's slots to weights in place (the indices stay), and their sum.
+template <int J> __device__ __forceinline__ void slots_to_weights(const Step4& s, float& sum) {
+  float w[8], ws;
+  s4_weights<J>(s, w, ws);
+#pragma unroll
+  for (int t = 0; t < 8; ++t) s4_d(s, J, t) = w[t];
+  sum = ws;
+}
+
+// The rays of every work item walked, a ray per thread, a warp to an item, every
+// step from scratch for its 4 points together (ilc_walk4.cuh), until they end or
+// their steps suit the lists, to which they are then left. kIdx: the slots hold
+// indices (V > 1, or a value table); otherwise the particles' own values.
+template <bool kMulti, bool kIdx>
+__global__ void __launch_bounds__(kSlotThreads, kWalkBlocks)
+batched_walk_kernel(const __grid_constant__ BatchK a, const __grid_constant__ GridView g,
+                    const char4* __restrict__ spiral_g, uint32_t* __restrict__ flags,
+                    unsigned long long* __restrict__ stats) {
+  __shared__ char4 spiral[1000];
+  __shared__ SlotMem slot_mem;
+  __shared__ float slot_ws[kMulti ? 4 : 1][kSlotThreads];
+  __shared__ unsigned long long blk[7];  // as BlockMem::stats
+  if (threadIdx.x < 7) blk[threadIdx.x] = 0ull;
+  load_spiral(spiral, spiral_g);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float* wstate = kMulti ? a.walk_state + ((size_t)blockIdx.x * kSlotThreads +
+                                           (size_t)warp * 32) * 4 * (size_t)a.V
+                         : nullptr;
+  for (;;) {
+    unsigned long long turn = 0;
+    if (lane == 0) turn = atomicAdd(a.queue + 1, 1ull);
+    turn = __shfl_sync(kAll, turn, 0);
+    if (turn >= a.n_items) break;
+    const uint64_t item = a.order ? (uint64_t)a.order[turn] : turn;
+    const JobDev& J = a.jobs[find_job(a.jobs, a.n_jobs, item)];
+    int ix, iy;
+    const bool inside = item_pixel(a, J, item, lane, ix, iy);
+    bool masked = true;
+    float o[3] = {0.0f, 0.0f, 0.0f}, len = 0.0f;
+    if (inside) ray_span(J, ix, iy, masked, o, len);
+    const float lx = J.look[0], ly = J.look[1], lz = J.look[2];
+    bool run = inside && !masked, leave = false;
+    float z = 0.0f, h = 1.0f, I = 0.0f, k1 = 0.0f;
+    uint32_t rs = 0, ra = 0;
+    WalkStats ws;
+    Pace pace = pace_start(0.0f);
+    if (kMulti) {
+      for (int i = lane; i < 32 * 4 * a.V; i += 32) wstate[i] = 0.0f;
+      __syncwarp();
+    }
+    while (__any_sync(kAll, run && z < len)) {
+      if (run && z < len && (int64_t)rs >= a.max_steps) {
+        atomicAdd(&blk[6], 1ull);
+        run = false;
+      }
+      const bool go = run && z < len;
+      ws.scans = 0;
+      if (go) {
+        float pts[4];
+        rkf_points(z, h, pts);
+        if (!kMulti) {
+          float e[4];
+          nn8_step4<kIdx>(g, spiral, slot_mem, o[0], o[1], o[2], lx, ly, lz, pts, e, ws);
+          const float zb = z;
+          rkf_advance_fp64(I, z, h, k1, a.atol, a.rtol, len, e, kEps, kHmin, kHmax, pts);
+          ++rs;
+          if (z != zb) ++ra;
+        } else {
+          Step4 s;
+          s4_bind(s, slot_mem);
+          nn8_walk_step4<true>(g, spiral, o[0], o[1], o[2], lx, ly, lz, pts, s, ws);
+          slots_to_weights<0>(s, slot_ws[0][threadIdx.x]);
+          slots_to_weights<1>(s, slot_ws[kMulti ? 1 : 0][threadIdx.x]);
+          slots_to_weights<2>(s, slot_ws[kMulti ? 2 : 0][threadIdx.x]);
+          slots_to_weights<3>(s, slot_ws[kMulti ? 3 : 0][threadIdx.x]);
+        }
+      }
+      if (kMulti) {
+        __syncwarp();
+        unsigned gom = __ballot_sync(kAll, go);
+        bool my_acc = false;
+        double my_nh = 0.0;
+        while (gom) {
+          const int r = __ffs(gom) - 1;
+          gom &= gom - 1;
+          const float zr = __shfl_sync(kAll, z, r), hr = __shfl_sync(kAll, h, r);
+          double nh;
+          const bool accept =
+              channels_step(a, WalkHand{slot_mem, slot_ws, warp * 32 + r},
+                            wstate + (size_t)r * 4 * a.V, zr, hr, lane, nh);
+          if (lane == r) {
+            my_acc = accept;
+            my_nh = nh;
+          }
+        }
+        __syncwarp();
+        if (go) {
+          const float znew = z + h;
+          if (my_acc) z = znew;
+          h = (float)my_nh;
+          if (z + h >= len) h = len - z + kEps;
+          ++rs;
+          if (my_acc) ++ra;
+        }
+      }
+      if (go && pace_slow(pace, a.leave, z, len, h, rs, ws.scans) && z < len) {
+        leave = true;
+        run = false;
+      }
+    }
+    mark_left(a.leave, inside && !masked, leave, 32 * turn + lane, lane);
+    if (!kMulti) {
+      if (inside && !leave)
+        a.out[J.out_offset + (size_t)iy * J.nx + ix] = masked ? 0.0f : I * J.scale;
+    } else {
+      const size_t plane = (size_t)J.nx * (size_t)J.ny;
+      for (int r = 0; r < 32; ++r) {
+        const int ixr = __shfl_sync(kAll, ix, r), iyr = __shfl_sync(kAll, iy, r);
+        const bool out_r = __shfl_sync(kAll, inside && !leave, r),
+                   m_r = __shfl_sync(kAll, masked, r);
+        if (!out_r) continue;
+        const float* Is = wstate + (size_t)r * 4 * a.V;
+        for (int c = lane; c < a.V; c += 32)
+          a.out[J.out_offset + (size_t)c * plane + (size_t)iyr * J.nx + ixr] =
+              m_r ? 0.0f : Is[c] * J.scale;
+      }
+      __syncwarp();
+    }
+    if (!leave) {
+      atomicAdd(&blk[0], (unsigned long long)rs);
+      atomicAdd(&blk[1], (unsigned long long)ra);
+      atomicAdd(&blk[3], (unsigned long long)ws.cells);
+      atomicAdd(&blk[4], (unsigned long long)ws.cands);
+      atomicMax(&blk[5], (unsigned long long)rs);
+    }
+    __syncwarp();
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    if (blk[6]) atomicOr(flags, FLAG_STEP_LIMIT);
+    atomicAdd(&stats[0], blk[0]);
+    atomicAdd(&stats[1], blk[1]);
+    atomicAdd(&stats[2], 4ull * blk[0]);
+    atomicAdd(&stats[3], blk[3]);
+    atomicAdd(&stats[4], blk[4]);
+    atomicMax(&stats[5], blk[5]);
+    atomicAdd(&stats[6], blk[6]);
   }
 }
 
@@ -513,10 +705,35 @@ cudaError_t launch_variant(Context& c, const BatchK& k, const GridView& g, int b
   return cudaGetLastError();
 }
 
-cudaError_t enqueue(Context& c, const BatchK& k, const GridView& g, int blocks) {
+// The walk kernel for these channels, and its resident blocks.
+using WalkKernel = void (*)(BatchK, GridView, const char4*, uint32_t*, unsigned long long*);
+WalkKernel walk_kernel(const BatchK& k, const GridView& g) {
+  return k.V > 1  ? batched_walk_kernel<true, true>
+         : g.vals ? batched_walk_kernel<false, true>
+                  : batched_walk_kernel<false, false>;
+}
+cudaError_t walk_blocks(const Context& c, WalkKernel kernel, int occ, int* blocks) {
+  int sms = 0, per_sm = 0;
+  cudaError_t e;
+  if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c.device)) ||
+      (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kSlotThreads, 0)))
+    return e;
+  if (occ > 0) per_sm = std::min(per_sm, occ);
+  *blocks = sms * std::max(per_sm, 1);
+  return cudaSuccess;
+}
+
+// blocks_w: of the walk in front (0: none).
+cudaError_t enqueue(Context& c, const BatchK& k, const GridView& g, int blocks, int blocks_w) {
   cudaError_t e;
   if ((e = cudaMemsetAsync(c.flags.p, 0, kFlagsBytes, c.stream))) return e;
-  if ((e = cudaMemsetAsync(c.queue.p, 0, 8, c.stream))) return e;
+  if ((e = cudaMemsetAsync(c.queue.p, 0, kQueueBytes, c.stream))) return e;
+  if (blocks_w > 0) {
+    walk_kernel(k, g)<<<blocks_w, kSlotThreads, 0, c.stream>>>(
+        k, g, c.spiral.as<char4>(), c.flags.as<uint32_t>(),
+        reinterpret_cast<unsigned long long*>(c.flags.as<char>() + 64));
+    if ((e = cudaGetLastError()) || (e = left_list_launch(c, k.leave))) return e;
+  }
   return k.V == 1 ? launch_variant<false>(c, k, g, blocks)
                   : launch_variant<true>(c, k, g, blocks);
 }
@@ -598,12 +815,25 @@ cudaError_t batched_launch(Context& c, const BatchArgs& a, float* kernel_ms) {
   k.over = c.list_over.as<float4>();
   GridView g = make_grid_view(c);
   if (a.V == 1) g.vals = a.chan;
+  // many rays: walked first, the lists get those that the walk leaves
+  int blocks_w = 0;
+  k.leave = walk_rule(c, a.rays, 32 * a.n_items, k.queue);
+  if (k.leave.left) {
+    if ((e = walk_blocks(c, walk_kernel(k, g), a.occupancy, &blocks_w))) return e;
+    if (a.V > 1 && c.walk_state.ensure((size_t)blocks_w * kSlotThreads * 4 * (size_t)k.V * 4)) {
+      cudaGetLastError();  // (no memory for the channels' states: lists for all rays)
+      k.leave.left = nullptr;
+      blocks_w = 0;
+    }
+    k.walk_state = c.walk_state.as<float>();
+  }
   if (!c.ev0) {
     if ((e = cudaEventCreate(&c.ev0)) || (e = cudaEventCreate(&c.ev1))) return e;
   }
   std::string key(reinterpret_cast<const char*>(&k), sizeof(k));
   key.append(reinterpret_cast<const char*>(&g), sizeof(g));
   key.append(reinterpret_cast<const char*>(&blocks), sizeof(blocks));
+  key.append(reinterpret_cast<const char*>(&blocks_w), sizeof(blocks_w));
   if (!c.batch_exec || key != c.batch_key) {
     if (c.batch_exec) {
       cudaGraphExecDestroy(c.batch_exec);
@@ -612,7 +842,7 @@ cudaError_t batched_launch(Context& c, const BatchArgs& a, float* kernel_ms) {
     c.batch_key.clear();
     cudaGraph_t graph = nullptr;
     if ((e = cudaStreamBeginCapture(c.stream, cudaStreamCaptureModeThreadLocal))) return e;
-    const cudaError_t el = enqueue(c, k, g, blocks);
+    const cudaError_t el = enqueue(c, k, g, blocks, blocks_w);
     e = cudaStreamEndCapture(c.stream, &graph);
     if (el) {
       if (graph) cudaGraphDestroy(graph);
@@ -628,7 +858,7 @@ cudaError_t batched_launch(Context& c, const BatchArgs& a, float* kernel_ms) {
     c.batch_key = key;
   }
   cudaEventRecord(c.ev0, c.stream);
-  ++c.launches;
+  c.launches += blocks_w > 0 ? 3 : 1;
   if ((e = cudaGraphLaunch(c.batch_exec, c.stream))) return e;
   cudaEventRecord(c.ev1, c.stream);
   if (kernel_ms) {

@@ -220,6 +220,7 @@ ilc_status batched_jobs(Context& c, int32_t V, const ilc_job* jobs, int32_t n_jo
   std::vector<JobDev> jd((size_t)n_jobs);
   const int tw = c.batch_tile_w, th = c.batch_tile_w > 0 ? 32 / c.batch_tile_w : 1;
   uint64_t items = 0;
+  double rays = 0.0;
   for (int32_t k = 0; k < n_jobs; ++k) {
     const ilc_job& j = jobs[k];
     if (!camera_ok(&j.camera)) return fail(c, ILC_ERR_INVALID_ARGUMENT, "invalid job camera");
@@ -262,6 +263,8 @@ ilc_status batched_jobs(Context& c, int32_t V, const ilc_job* jobs, int32_t n_jo
     d.scale = j.scale;
     d.out_offset = j.out_offset;
     d.item_begin = items;
+    const double r = d.aperture / d.ps_d;  // the aperture's radius in pixels
+    rays += d.aperture > 0.0 ? std::min((double)npix, 3.14159265 * r * r) : (double)npix;
     items += tw > 0 ? (uint64_t)d.tiles_x * (uint64_t)((d.ny + th - 1) / th)
                     : (uint64_t)d.tiles_x;
   }
@@ -271,6 +274,7 @@ ilc_status batched_jobs(Context& c, int32_t V, const ilc_job* jobs, int32_t n_jo
   a->jobs = c.jobs.as<JobDev>();
   a->n_jobs = n_jobs;
   a->n_items = items;
+  a->rays = rays;
   a->V = V;
   a->chan = nullptr;
   a->atol = tol.absolute;
@@ -486,7 +490,7 @@ void ilc_destroy(ilc_ctx* h) {
   Context& c = h->c;
   cudaSetDevice(c.device);
   if (c.stream) cudaStreamSynchronize(c.stream);
-  for (DevBuf* b : {&c.tile_queue, &c.list_over, &c.query_sort, &c.parts, &c.cells, &c.s2u, &c.keys_a, &c.keys_b, &c.vals_a, &c.vals_b,
+  for (DevBuf* b : {&c.tile_queue, &c.list_over, &c.rays_left, &c.walk_state, &c.query_sort, &c.parts, &c.cells, &c.s2u, &c.keys_a, &c.keys_b, &c.vals_a, &c.vals_b,
                     &c.hist, &c.tmp_in, &c.gaunt, &c.gaunt_pad, &c.list_d, &c.list_v, &c.list_id, &c.in_a,
                     &c.in_b, &c.in_c, &c.out_a, &c.out_b, &c.out_c, &c.spiral, &c.flags,
                     &c.rec_h, &c.rec_n, &c.adj_dT, &c.adj_dR, &c.adj_grad, &c.adj_seed,

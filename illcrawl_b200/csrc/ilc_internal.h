@@ -45,6 +45,27 @@ struct GridParams {
   uint64_t total;
 };
 
+// Launches of many adaptive rays walk first (ilc_walk4.cuh) and leave rays to the
+// candidate lists by this rule.
+struct LeaveRule {
+  // Walk and lists take the same time for steps of `even / (rays - line)` (with
+  // fewer rays than `line` lists are always ahead), and with the chip full of
+  // short ones, `least`.
+  float even, line, least;
+  float rays;                // of the launch, without masked ones
+  unsigned long long* done;  // of them, ended or left
+  uint8_t* left;             // a bit per ray: left to the lists (nullptr: nothing is walked)
+  uint64_t n_marks;
+  uint32_t* list;            // the rays left, in their order
+  uint32_t* n_left;
+};
+
+// Where there are more rays than kWalkRays times the line, and memory for the marks
+// and the list, walk_rule() sets `left`. The queue of such a launch: counters of the
+// lists and the walk, rays done, rays left.
+constexpr double kWalkRays = 3.75;
+constexpr size_t kQueueBytes = 32;
+
 struct Context {
   int device = 0;
   cudaStream_t stream = nullptr;
@@ -91,6 +112,9 @@ struct Context {
   DevBuf in_a, in_b, in_c, out_a, out_b, out_c;
   DevBuf tile_queue;  // render and adjoint kernels: ray counter
   DevBuf list_over;   // ray kernels: candidate lists beyond shared memory
+  DevBuf walk_state;  // batched walk: the rays' channel states
+  DevBuf rays_left;   // ray kernels: rays that the walk left to the lists: a bit each, list
+  LeaveRule leave = {};  // of the last render: which rays it walked
   DevBuf spiral;     // char4[1000]
   DevBuf flags;      // uint32 error flags + uint64 stats
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -238,6 +262,10 @@ cudaError_t adjoint_ray_launch(Context& c, const RenderArgs& a, int mode, const 
 cudaError_t adjoint_chain_launch(Context& c, const double* grad, uint64_t n, const float* dq_lnrho,
                                  const float* dq_lnT, float* g_lnrho, float* g_lnT);
 cudaError_t render_launch(Context& c, const RenderArgs& a, float* kernel_ms);
+LeaveRule walk_rule(Context& c, double rays, unsigned long long n_rays,
+                    unsigned long long* queue);
+// The list of the rays marked, in their order.
+cudaError_t left_list_launch(Context& c, const LeaveRule& r);
 
 // One camera of a batched render, as the kernel reads it.
 struct JobDev {
@@ -257,6 +285,7 @@ struct BatchArgs {
   const JobDev* jobs;     // device
   int32_t n_jobs;
   uint64_t n_items;
+  double rays;            // inside the apertures
   int32_t V;
   const float* chan;      // device, sorted order, n x V (V = 1: nullptr = particles' q)
   float* out;             // device images

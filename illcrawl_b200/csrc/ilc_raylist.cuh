@@ -49,10 +49,9 @@
 // arithmetic with 4 warps per scheduler (stalls of 2.3 cycles per issue) and
 // instruction fetch (2.0); the grid stays in L2 (DRAM 2 MB read per launch).
 // Images of very many rays gain less, since there the walks from scratch filled
-// the chip too: 1024^2 band map of 4,194,304 cells, 6 Mpc: 12.16 -> 10.77 s; and
-// loose tolerances away from dense cores, whose steps are long, lose: 256^2 /
-// 1024^2 projection of 262,144 cells through the outer 500 kpc at rtol 1e-2:
-// 3.3 -> 5.6 / 19 -> 81 ms (through the core, 2 Mpc, 256^2: 554 -> 44 ms).
+// the chip too: 1024^2 band map of 4,194,304 cells, 6 Mpc: 12.16 -> 10.77 s. Steps
+// that are long against a cell use a list once or twice, and lose: launches of many
+// rays walk those (ilc_walk4.cuh).
 #pragma once
 
 #include "ilc_device.cuh"

@@ -3,8 +3,9 @@
 // volumetric_integration.cpp:32-88) as one kernel launch.
 //
 // Four lanes own one pixel's integrator and run its RKF4(5) steps to the end of
-// the ray, one lane per integrand point (ilc_raylist.cuh); fixed steps that are
-// long against a cell are walked one ray per thread (ilc_walk4.cuh). A ray's
+// the ray, one lane per integrand point (ilc_raylist.cuh); steps that are long
+// against a cell are walked one ray per thread (ilc_walk4.cuh): fixed ones by a
+// rule on the launch, adaptive ones as far as each ray's steps stay long. A ray's
 // state depends only on its own evaluations, so this is the same computation as
 // the reference's lock-step loop with stream compaction, without its
 // per-iteration host synchronisations.
@@ -72,6 +73,7 @@ struct RenderK {
   unsigned long long n_rays;  // 128 per 16 x 8 tile
   unsigned tiles_x;
   float4* over;               // list overflow, kOver per resident ray
+  LeaveRule leave;            // rays walked first, and those left to the lists
 };
 
 constexpr int kRenderBlocks = 4;  // per SM, by registers and shared memory
@@ -127,9 +129,9 @@ render_kernel(const __grid_constant__ RenderK a, const __grid_constant__ GridVie
       const unsigned long long q = take_rays(a.queue, want, fresh, lane, wg);
       fresh = false;
       if (!have && !drained) {
-        drained = q >= a.n_rays;
+        drained = q >= list_rays(a.leave, a.n_rays);
         if (!drained) {
-          ray_pixel(a, q, ix, iy);
+          ray_pixel(a, list_ray(a.leave, q), ix, iy);
           have = ix < a.cam.nx && iy < a.row_end;
         }
         if (have) {
@@ -236,87 +238,140 @@ render_kernel(const __grid_constant__ RenderK a, const __grid_constant__ GridVie
   }
 }
 
-// Pixel of this thread in the 16 x 8 tile (bx, by): each warp an 8 x 4 tile, so
-// its 32 rays are neighbours.
-__device__ __forceinline__ void walk_pixel(const RenderK& a, int bx, int by, int& ix, int& iy) {
-  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
-  ix = bx * kTileX + (warp & 1) * 8 + (lane & 7);
-  iy = a.row0 + by * a.row_stride * kTileY + (warp >> 1) * 4 + (lane >> 3);
-}
-
-// Fixed steps of one 16 x 8 tile of rays, a ray per thread, every step walked
-// from scratch for its 4 points together (ilc_walk4.cuh): I += delta4.
+// The rays of one tile, a ray per thread, every step walked from scratch for its 4
+// points together (ilc_walk4.cuh). kFixed: uniform frozen steps; otherwise frozen
+// per-ray sequences or adaptive steps, as in render_kernel, and rays whose steps
+// suit the lists are left.
+template <bool kFixed>
 __device__ __forceinline__ void walk_tile(const RenderK& a, const GridView& g,
                                           const char4* __restrict__ spiral, SlotMem& slot_mem,
-                                          unsigned long long* __restrict__ stats, int bx, int by) {
+                                          uint32_t* __restrict__ flags,
+                                          unsigned long long* __restrict__ stats,
+                                          unsigned long long tile) {
+  const unsigned long long q = 128 * tile + walk_ray();
   int ix, iy;
-  walk_pixel(a, bx, by, ix, iy);
+  ray_pixel(a, q, ix, iy);
   const bool active = ix < a.cam.nx && iy < a.row_end;
   WalkStats ws;
-  unsigned long long steps = 0;
+  unsigned long long steps = 0, acc = 0, at_limit = 0;
+  bool leave = false;
   if (active) {
     float px, py, pz, pts[4];
     pixel_corner(a.cam, ix, iy, px, py, pz);
-    float I = 0.0f, z = a.z0, k1 = 0.0f;
-    const float h = a.fixed_h;
+    const int64_t lray = (int64_t)(iy - a.row0) * a.cam.nx + ix;  // in the launch's rows
+    float I = 0.0f, z = a.z0, h = kFixed ? a.fixed_h : 1.0f, k1 = 0.0f;
+    const float fa = (float)a.atol, fr = (float)a.rtol;
     double Id = 0.0;  // out_d: the same increments summed in double
-    for (int64_t s = 0; s < a.fixed_steps; ++s) {
+    const bool frozen = kFixed || a.replay_h;
+    int64_t limit = kFixed ? a.fixed_steps : a.max_steps;
+    const float* hs = nullptr;
+    if (!kFixed && a.replay_h) {
+      const int64_t nr = a.replay_n[lray];
+      limit = nr < 0 ? 0 : (nr > a.rec_cap ? a.rec_cap : nr);
+      hs = a.replay_h + lray * a.rec_cap;
+    }
+    Pace pace = pace_start(z);
+    while ((int64_t)steps < limit && (frozen || z < a.z_end)) {
+      if (!kFixed && hs) h = hs[steps];
+      ws.scans = 0;
       rkf_points(z, h, pts);
       float e[4];
-      nn8_step4(g, spiral, slot_mem, px, py, pz, a.cam.look0, a.cam.look1, a.cam.look2, pts, e,
-                ws);
-      float d4 = 25.f / 216.f * k1 + 1408.f / 2565.f * e[0] + 2197.f / 4101.f * e[1] -
-                 1.f / 5.f * e[2];
-      d4 *= h;
-      I = I + d4;
-      if (a.out_d) Id += (double)d4;
-      z += h;
-      k1 = e[2];
+      nn8_step4<false>(g, spiral, slot_mem, px, py, pz, a.cam.look0, a.cam.look1, a.cam.look2,
+                       pts, e, ws);
+      ++steps;
+      if (frozen) {
+        // every step accepted, I += delta4
+        float d4 = 25.f / 216.f * k1 + 1408.f / 2565.f * e[0] + 2197.f / 4101.f * e[1] -
+                   1.f / 5.f * e[2];
+        d4 *= h;
+        I = I + d4;
+        if (a.out_d) Id += (double)d4;
+        z += h;
+        k1 = e[2];
+        ++acc;
+      } else {
+        const float zb = z, hb = h;
+        if (a.controller == ILC_CONTROLLER_REF32)
+          rkf_advance_ref32(I, z, h, k1, fa, fr, a.z_end, e, kEps, kHmin, kHmax, pts);
+        else
+          rkf_advance_fp64(I, z, h, k1, a.atol, a.rtol, a.z_end, e, kEps, kHmin, kHmax, pts);
+        if (z != zb) {
+          if (a.rec_h && (int64_t)acc < a.rec_cap)
+            a.rec_h[lray * a.rec_cap + (int64_t)acc] = hb;
+          ++acc;
+        }
+      }
+      if (!kFixed && a.leave.left &&
+          pace_slow(pace, a.leave, z, a.z_end, h, steps, ws.scans) &&
+          (int64_t)steps < limit && (frozen || z < a.z_end)) {
+        leave = true;
+        break;
+      }
     }
-    steps = (unsigned long long)a.fixed_steps;
-    const size_t pix = (size_t)iy * a.cam.nx + ix;
-    if (a.out) a.out[pix] = a.apply_scale ? I * a.scale : I;
-    if (a.out_d) a.out_d[pix] = a.apply_scale ? Id * (double)a.scale : Id;
-    if (a.ray_stats) {
-      uint64_t* q = a.ray_stats + 4 * ((int64_t)(iy - a.row0) * a.cam.nx + ix);
-      q[0] = q[1] = steps;
-      q[2] = ws.cells;
-      q[3] = ws.cands;
+    if (leave) {
+      steps = acc = 0;
+      ws = WalkStats();
+    } else {
+      const size_t pix = (size_t)iy * a.cam.nx + ix;
+      if (a.out) a.out[pix] = a.apply_scale ? I * a.scale : I;
+      if (a.out_d) a.out_d[pix] = a.apply_scale ? Id * (double)a.scale : Id;
+      if (!frozen && a.rec_n) {
+        a.rec_n[lray] = (int32_t)min((int64_t)acc, a.rec_cap);
+        if ((int64_t)acc > a.rec_cap) atomicOr(flags, FLAG_REC_OVERFLOW);
+      }
+      if (a.ray_stats) {
+        uint64_t* rs = a.ray_stats + 4 * lray;
+        rs[0] = steps;
+        rs[1] = acc;
+        rs[2] = ws.cells;
+        rs[3] = ws.cands;
+      }
+      if (!frozen && z < a.z_end) {
+        at_limit = 1;
+        atomicOr(flags, FLAG_STEP_LIMIT);
+      }
     }
   }
+  const int lane = threadIdx.x & 31;
+  if (!kFixed && a.leave.left) mark_left(a.leave, active, leave, q, lane);
   unsigned long long cells = ws.cells, cands = ws.cands, sum = steps, most = steps;
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) {
     cells += __shfl_xor_sync(kAll, cells, off);
     cands += __shfl_xor_sync(kAll, cands, off);
     sum += __shfl_xor_sync(kAll, sum, off);
+    acc += __shfl_xor_sync(kAll, acc, off);
+    at_limit += __shfl_xor_sync(kAll, at_limit, off);
     most = max(most, __shfl_xor_sync(kAll, most, off));
   }
-  if ((threadIdx.x & 31) == 0) {
+  if (lane == 0) {
     atomicAdd(&stats[0], sum);
-    atomicAdd(&stats[1], sum);
+    atomicAdd(&stats[1], acc);
     atomicAdd(&stats[2], 4ull * sum);
     atomicAdd(&stats[3], cells);
     atomicAdd(&stats[4], cands);
     atomicMax(&stats[5], most);
+    if (at_limit) atomicAdd(&stats[6], at_limit);
   }
 }
 
 // The resident blocks take tiles row by row from the queue until none is left.
+template <bool kFixed>
 __global__ void __launch_bounds__(kSlotThreads, kRenderBlocks)
 walk_kernel(const __grid_constant__ RenderK a, const __grid_constant__ GridView g,
-            const char4* __restrict__ spiral_g, unsigned long long* __restrict__ stats) {
+            const char4* __restrict__ spiral_g, uint32_t* __restrict__ flags,
+            unsigned long long* __restrict__ stats) {
   __shared__ char4 spiral[1000];
   __shared__ SlotMem slot_mem;
   __shared__ unsigned long long next_tile;
   load_spiral(spiral, spiral_g);
   for (;;) {
-    if (threadIdx.x == 0) next_tile = atomicAdd(a.queue, 1ull);
+    if (threadIdx.x == 0) next_tile = atomicAdd(a.queue + 1, 1ull);
     __syncthreads();
     const unsigned long long t = next_tile;
     __syncthreads();
     if (128 * t >= a.n_rays) break;
-    walk_tile(a, g, spiral, slot_mem, stats, (int)(t % a.tiles_x), (int)(t / a.tiles_x));
+    walk_tile<kFixed>(a, g, spiral, slot_mem, flags, stats, t);
   }
 }
 
@@ -332,12 +387,75 @@ walk_kernel(const __grid_constant__ RenderK a, const __grid_constant__ GridView 
 // 400^2 33 / 157 / 391 against 7.8 / 65 / 420; 1024^2 200 / 948 / 2371 against
 // 22 / 185 / 1304. With 20,000 cells the slowest warp is shorter and the walk is
 // ahead from half as many rays (150^2, 32 steps: 9.3 against 4.7 ms).
-static bool render_walks(const Context& c, const RenderArgs& a) {
-  if (a.fixed_steps <= 0 || a.replay_h) return false;
-  const double rays = (double)a.nx * (double)(a.rows > 0 ? a.rows : a.ny);
+//
+// Adaptive rays leave the walk below that length, with the rays that are still
+// under way for the rays (LeaveRule).
+LeaveRule walk_rule(Context& c, double rays, unsigned long long n_rays,
+                    unsigned long long* queue) {
   const double cell = ((double)c.gp.cs[0] + c.gp.cs[1] + c.gp.cs[2]) / 3.0;
   const double line = 16384.0 * std::fmin(1.0, std::pow((double)c.n_particles / 1048576.0, 0.19));
-  return rays * a.fixed_h > line * (a.fixed_h + 0.28 * cell);
+  LeaveRule r;
+  std::memset(&r, 0, sizeof(r));  // padding too: the bytes key the batched launch graph
+  r.even = (float)(0.28 * cell * line);
+  r.line = (float)line;
+  r.least = (float)(0.01 * cell);
+  if (!(rays > kWalkRays * line) || n_rays > 0xffffffffull) return r;
+  const size_t marks = ((size_t)n_rays / 8 + 15) / 16 * 16;
+  if (c.rays_left.ensure(marks + 4 * (size_t)n_rays) != cudaSuccess) {
+    cudaGetLastError();  // (all rays take lists then)
+    return r;
+  }
+  r.rays = (float)rays;
+  r.n_marks = n_rays;
+  r.done = queue + 2;
+  r.n_left = reinterpret_cast<uint32_t*>(queue + 3);
+  r.left = c.rays_left.as<uint8_t>();
+  r.list = c.rays_left.as<uint32_t>() + marks / 4;
+  return r;
+}
+
+namespace {
+
+// The numbers of the marked rays in their order, by one block: 4 us for 65,536 rays,
+// 11 us for 1,048,576.
+constexpr int kCompact = 1024;
+__global__ void __launch_bounds__(kCompact)
+left_list_kernel(const uint32_t* __restrict__ marks, uint32_t words, uint32_t* __restrict__ list,
+                 uint32_t* __restrict__ n_left) {
+  __shared__ uint32_t part[32];
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  uint32_t base = 0;
+  for (uint32_t w0 = 0; w0 < words; w0 += 4 * kCompact) {
+    uint32_t m[4], n = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < 4; ++k) {
+      const uint32_t w = w0 + 4 * threadIdx.x + k;
+      m[k] = w < words ? marks[w] : 0u;
+      n += __popc(m[k]);
+    }
+    if (!__syncthreads_or((int)n)) continue;
+    const uint32_t incl = (uint32_t)warp_inclusive((int)n, (int)lane);
+    if (lane == 31) part[warp] = incl;
+    __syncthreads();
+    const uint32_t below = (uint32_t)warp_inclusive((int)part[lane], (int)lane);
+    uint32_t at = base + incl - n + (warp ? __shfl_sync(kAll, below, warp - 1) : 0u);
+#pragma unroll
+    for (uint32_t k = 0; k < 4; ++k) {
+      for (uint32_t b = m[k]; b; b &= b - 1)
+        list[at++] = 32 * (w0 + 4 * threadIdx.x + k) + __ffs(b) - 1;
+    }
+    base += __shfl_sync(kAll, below, 31);
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) *n_left = base;
+}
+
+}  // namespace
+
+cudaError_t left_list_launch(Context& c, const LeaveRule& r) {
+  left_list_kernel<<<1, kCompact, 0, c.stream>>>(reinterpret_cast<const uint32_t*>(r.left),
+                                                 (uint32_t)(r.n_marks / 32), r.list, r.n_left);
+  return cudaGetLastError();
 }
 
 cudaError_t render_launch(Context& c, const RenderArgs& a, float* kernel_ms) {
@@ -377,41 +495,60 @@ cudaError_t render_launch(Context& c, const RenderArgs& a, float* kernel_ms) {
       (unsigned long long)k.tiles_x * (unsigned)((tile_rows + k.row_stride - 1) / k.row_stride);
   k.n_rays = 128ull * tiles;
   if ((e = c.tile_queue.ensure(256))) return e;
-  if ((e = cudaMemsetAsync(c.tile_queue.p, 0, 8, c.stream))) return e;
+  if ((e = cudaMemsetAsync(c.tile_queue.p, 0, kQueueBytes, c.stream))) return e;
   k.queue = c.tile_queue.as<unsigned long long>();
-  const bool walk = render_walks(c, a);
+  // fixed steps: walk or lists; otherwise a walk of many rays and lists for those it leaves
+  const bool fixed = a.fixed_steps > 0 && !a.replay_h;
+  const double rays = (double)a.nx * (double)(k.row_end - k.row0) / (double)k.row_stride;
+  k.leave = walk_rule(c, fixed ? 0.0 : rays, k.n_rays, k.queue);
+  c.leave = k.leave;
+  const bool walks =
+      fixed ? (rays - k.leave.line) * a.fixed_h > k.leave.even : k.leave.left != nullptr;
+  const bool lists = !fixed || !walks;
   // as many blocks as are resident, or `occ` per SM
   const int occ = a.occupancy_override >= 0 ? a.occupancy_override : c.render_occupancy;
-  int sms = 0, per_sm = 0;
+  const auto walker = fixed ? walk_kernel<true> : walk_kernel<false>;
+  int sms = 0, per_sm = 0, per_sm_w = 0;
   if ((e = cudaFuncSetAttribute(render_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)sizeof(RenderMem))) ||
       (e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c.device)) ||
-      (e = walk ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, walk_kernel,
-                                                                kSlotThreads, 0)
-                : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, render_kernel,
-                                                                kListThreads,
-                                                                sizeof(RenderMem))))
+      (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_w, walker, kSlotThreads, 0)) ||
+      (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, render_kernel, kListThreads,
+                                                         sizeof(RenderMem))))
     return e;
-  if (occ > 0) per_sm = std::min(per_sm, occ);
-  // (down to one ray per warp: the rays of a small image build and replay their
-  // lists next to each other instead of in turn)
-  const unsigned blocks =
-      (unsigned)std::min<unsigned long long>((unsigned long long)sms * std::max(per_sm, 1),
-                                             walk ? tiles : 128 / kListWarps * tiles);
-  if (!walk && (e = c.list_over.ensure((size_t)blocks * kListWarps * kRays * kOver * 16))) return e;
+  if (occ > 0) {
+    per_sm = std::min(per_sm, occ);
+    per_sm_w = std::min(per_sm_w, occ);
+  }
+  // (lists: down to one ray per warp: the rays of a small image build and replay
+  // their lists next to each other instead of in turn)
+  const unsigned blocks = (unsigned)std::min<unsigned long long>(
+      (unsigned long long)sms * std::max(per_sm, 1), 128 / kListWarps * tiles);
+  const unsigned blocks_w = (unsigned)std::min<unsigned long long>(
+      (unsigned long long)sms * std::max(per_sm_w, 1), tiles);
+  if (lists && (e = c.list_over.ensure((size_t)blocks * kListWarps * kRays * kOver * 16))) return e;
   k.over = c.list_over.as<float4>();
   if (!c.ev0) {
     if ((e = cudaEventCreate(&c.ev0)) || (e = cudaEventCreate(&c.ev1))) return e;
   }
   cudaEventRecord(c.ev0, c.stream);
-  ++c.launches;
   unsigned long long* stats = reinterpret_cast<unsigned long long*>(c.flags.as<char>() + 64);
-  if (walk)
-    walk_kernel<<<blocks, kSlotThreads, 0, c.stream>>>(k, g, c.spiral.as<char4>(), stats);
-  else
+  if (walks) {
+    ++c.launches;
+    walker<<<blocks_w, kSlotThreads, 0, c.stream>>>(k, g, c.spiral.as<char4>(),
+                                                    c.flags.as<uint32_t>(), stats);
+    if ((e = cudaGetLastError())) return e;
+    if (lists) {
+      ++c.launches;
+      if ((e = left_list_launch(c, k.leave))) return e;
+    }
+  }
+  if (lists) {
+    ++c.launches;
     render_kernel<<<blocks, kListThreads, sizeof(RenderMem), c.stream>>>(
         k, g, c.spiral.as<char4>(), c.flags.as<uint32_t>(), stats);
-  if ((e = cudaGetLastError())) return e;
+    if ((e = cudaGetLastError())) return e;
+  }
   cudaEventRecord(c.ev1, c.stream);
   if (kernel_ms) {
     if ((e = cudaEventSynchronize(c.ev1))) return e;

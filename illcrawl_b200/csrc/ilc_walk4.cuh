@@ -13,14 +13,15 @@
 // the candidate loads (one 16-byte load serves four distance tests). Points in
 // a different cell or subcell are walked in a further pass.
 //
-// Used for fixed steps that are long against a cell over many rays, where a
-// candidate list (ilc_raylist.cuh) would serve too few steps: one walk costs about
-// the same whatever the step, and 32 neighbouring rays share its cells in L1
-// (1024^2 rays x 64 steps through 1,048,576 cells: 62 ms, with lists 558 ms).
+// Used for steps that are long against a cell over many rays, where a candidate
+// list (ilc_raylist.cuh) would serve too few steps: one walk costs about the same
+// whatever the step, and 32 neighbouring rays share its cells in L1 (1024^2 rays x
+// 64 fixed steps through 1,048,576 cells: 62 ms, with lists 558 ms).
 // Bound by instruction issue and, below some 20,000 rays, by the warp that
 // crosses the densest cells.
 #pragma once
 
+#include "ilc_internal.h"
 #include "ilc_raylist.cuh"
 
 namespace ilc {
@@ -146,27 +147,57 @@ __device__ __forceinline__ void s4_test(Step4& s, float& thr, float d2, float va
   }
 }
 
-template <int J> __device__ __forceinline__ float s4_finalize(const Step4& s) {
-  float w[8];
+// Weights of point J's slots (get_weight3d) and their sum, in slot order.
+template <int J> __device__ __forceinline__ void s4_weights(const Step4& s, float w[8], float& ws) {
 #pragma unroll
   for (int t = 0; t < 8; ++t) w[t] = weight3d(s4_d(s, J, t));
-  float ws = 0.0f;
+  ws = 0.0f;
 #pragma unroll
   for (int t = 0; t < 8; ++t) ws = ws + w[t];
-  float dot = 0.0f;
-#pragma unroll
-  for (int t = 0; t < 8; ++t) dot = __fmaf_rn(w[t], s4_v(s, J, t), dot);
-  float res = 0.0f;
-  if (ws != 0.0f && dot != 0.0f) res = dot / ws;
-  return res;
 }
 
-// Distance tests of one candidate against the active points.
-template <bool kSharedXY>
-__device__ __forceinline__ void cand_d2(const Step4& s, const float4& P, float d2[4]) {
+// Value of point J (finalize order). kIdx: the slots hold sorted indices, the
+// values are read from vals, or from the particles where that is null.
+template <int J, bool kIdx>
+__device__ __forceinline__ float s4_value(const GridView& g, const Step4& s) {
+  float w[8], ws;
+  s4_weights<J>(s, w, ws);
+  float dot = 0.0f;
+#pragma unroll
+  for (int t = 0; t < 8; ++t) {
+    float v = s4_v(s, J, t);
+    if (kIdx) {
+      const int id = __float_as_int(v);
+      v = id < 0 ? 0.0f : (g.vals ? __ldg(&g.vals[id]) : __ldg(&g.parts[id].w));
+    }
+    dot = __fmaf_rn(w[t], v, dot);
+  }
+  return (ws != 0.0f && dot != 0.0f) ? dot / ws : 0.0f;
+}
+
+__device__ __forceinline__ void cand_insert(Step4& s, float thr[4], const float d2[4],
+                                            float pay) {
+  s4_test<0>(s, thr[0], d2[0], pay);
+  s4_test<1>(s, thr[1], d2[1], pay);
+  s4_test<2>(s, thr[2], d2[2], pay);
+  s4_test<3>(s, thr[3], d2[3], pay);
+}
+
+// Candidate p against the active points; the slots take its value, or (kIdx) its
+// sorted index.
+// With a shared x/y part, every point's squared distance is fl(fxy + fz^2)
+// >= fxy (rounding is monotone and fz^2 >= 0), so a candidate whose fxy
+// exceeds the largest threshold thrmax cannot be inserted for any point.
+// thrmax may be stale (larger than the current thresholds): the test only
+// skips work that could not insert.
+template <bool kSharedXY, bool kIdx>
+__device__ __forceinline__ void test_candidate(Step4& s, float thr[4], float thrmax,
+                                               const float4& P, int p) {
+  float d2[4];
   if (kSharedXY) {
     const float fx = P.x - s.qx[0], fy = P.y - s.qy[0];
     const float fxy = fx * fx + fy * fy;
+    if (fxy > thrmax) return;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const float fz = P.z - s.qz[j];
@@ -179,46 +210,7 @@ __device__ __forceinline__ void cand_d2(const Step4& s, const float4& P, float d
       d2[j] = (fx * fx + fy * fy) + fz * fz;
     }
   }
-}
-
-__device__ __forceinline__ void cand_insert(Step4& s, float thr[4], const float d2[4],
-                                            const float4& P) {
-  const float pay = P.w;
-  s4_test<0>(s, thr[0], d2[0], pay);
-  s4_test<1>(s, thr[1], d2[1], pay);
-  s4_test<2>(s, thr[2], d2[2], pay);
-  s4_test<3>(s, thr[3], d2[3], pay);
-}
-
-template <bool kSharedXY>
-__device__ __forceinline__ void test_candidate(Step4& s, float thr[4], const float4& P) {
-  float d2[4];
-  cand_d2<kSharedXY>(s, P, d2);
-  cand_insert(s, thr, d2, P);
-}
-
-// With a shared x/y part, every point's squared distance is fl(fxy + fz^2)
-// >= fxy (rounding is monotone and fz^2 >= 0), so a candidate whose fxy
-// exceeds the largest threshold thrmax cannot be inserted for any point.
-// thrmax may be stale (larger than the current thresholds): the test only
-// skips work that could not insert.
-template <bool kSharedXY>
-__device__ __forceinline__ void test_candidate_xy(Step4& s, float thr[4], float thrmax,
-                                                  const float4& P) {
-  if (kSharedXY) {
-    const float fx = P.x - s.qx[0], fy = P.y - s.qy[0];
-    const float fxy = fx * fx + fy * fy;
-    if (fxy > thrmax) return;
-    float d2[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float fz = P.z - s.qz[j];
-      d2[j] = fxy + fz * fz;
-    }
-    cand_insert(s, thr, d2, P);
-  } else {
-    test_candidate<false>(s, thr, P);
-  }
+  cand_insert(s, thr, d2, kIdx ? __int_as_float(p) : P.w);
 }
 
 // Cells with more candidates than this are scanned through their sub-box codes.
@@ -249,7 +241,7 @@ __device__ __forceinline__ bool prune_range(const GridView& g, int ix, int iy, i
 // axis), so the x/y part of every squared distance, (dx*dx + dy*dy), is one
 // value for the 4 points and is evaluated once -- the same operations in the
 // same order, hence the same bits, as evaluating it per point.
-template <bool kSharedXY>
+template <bool kSharedXY, bool kIdx>
 __device__ __forceinline__ void walk4(const GridView& g, const char4* __restrict__ spiral,
                                       Step4& s, unsigned mask, int cx, int cy, int cz, int sub,
                                       WalkStats& st) {
@@ -324,6 +316,7 @@ __device__ __forceinline__ void walk4(const GridView& g, const char4* __restrict
                              0.0f);
       if ((gx * gx + gy * gy) + gz * gz > thrmax) continue;
     }
+    st.scans += be.y - be.x > kPruneMin ? (uint32_t)(be.y - be.x) >> 2 : (uint32_t)(be.y - be.x);
     if (be.y - be.x > kPruneMin) {
       // Dense cell: candidates in ascending index order, 8 codes per load. The
       // range follows the search radius as it shrinks while the cell is scanned
@@ -344,7 +337,7 @@ __device__ __forceinline__ void walk4(const GridView& g, const char4* __restrict
         while (hits) {
           const int p = pw + __ffs(hits) - 1;
           hits &= hits - 1;
-          test_candidate_xy<kSharedXY>(s, thr, thrmax, __ldg(&g.parts[p]));
+          test_candidate<kSharedXY, kIdx>(s, thr, thrmax, __ldg(&g.parts[p]), p);
         }
       }
       continue;
@@ -352,13 +345,14 @@ __device__ __forceinline__ void walk4(const GridView& g, const char4* __restrict
     float4 P = __ldg(&g.parts[be.x]);
     for (int p = be.x; p < be.y; ++p) {
       const float4 N = (p + 1 < be.y) ? __ldg(&g.parts[p + 1]) : P;  // prefetch
-      test_candidate_xy<kSharedXY>(s, thr, thrmax, P);
+      test_candidate<kSharedXY, kIdx>(s, thr, thrmax, P, p);
       P = N;
     }
   }
 }
 
 // nn8 walk of the 4 points of one step; the slots are left in s.
+template <bool kIdx>
 __device__ __forceinline__ void nn8_walk_step4(const GridView& g,
                                                const char4* __restrict__ spiral, float px,
                                                float py, float pz, float lx, float ly, float lz,
@@ -391,7 +385,7 @@ __device__ __forceinline__ void nn8_walk_step4(const GridView& g,
     sb[j] = sx + 2 * sy + 4 * sz;
   }
   s.crad = g.cell_radius;
-  const float empty = 0.0f;
+  const float empty = kIdx ? __int_as_float(-1) : 0.0f;
   s4_init<0>(s, empty);
   s4_init<1>(s, empty);
   s4_init<2>(s, empty);
@@ -409,25 +403,108 @@ __device__ __forceinline__ void nn8_walk_step4(const GridView& g,
       if (((todo >> j) & 1u) && cx[j] == c0x && cy[j] == c0y && cz[j] == c0z && sb[j] == s0)
         mask |= 1u << j;
     if (shared_xy)
-      walk4<true>(g, spiral, s, mask, c0x, c0y, c0z, s0, st);
+      walk4<true, kIdx>(g, spiral, s, mask, c0x, c0y, c0z, s0, st);
     else
-      walk4<false>(g, spiral, s, mask, c0x, c0y, c0z, s0, st);
+      walk4<false, kIdx>(g, spiral, s, mask, c0x, c0y, c0z, s0, st);
     todo &= ~mask;
   }
 }
 
 // nn8 values of the 4 points of one step (e[j] for point j).
+template <bool kIdx>
 __device__ __forceinline__ void nn8_step4(const GridView& g, const char4* __restrict__ spiral,
                                           SlotMem& sm, float px, float py, float pz, float lx,
                                           float ly, float lz, const float zq[4], float e[4],
                                           WalkStats& st) {
   Step4 s;
   s4_bind(s, sm);
-  nn8_walk_step4(g, spiral, px, py, pz, lx, ly, lz, zq, s, st);
-  e[0] = s4_finalize<0>(s);
-  e[1] = s4_finalize<1>(s);
-  e[2] = s4_finalize<2>(s);
-  e[3] = s4_finalize<3>(s);
+  nn8_walk_step4<kIdx>(g, spiral, px, py, pz, lx, ly, lz, zq, s, st);
+  e[0] = s4_value<0, kIdx>(g, s);
+  e[1] = s4_value<1, kIdx>(g, s);
+  e[2] = s4_value<2, kIdx>(g, s);
+  e[3] = s4_value<3, kIdx>(g, s);
+}
+
+// ---------------------------------------------------------------------------
+// Adaptive steps. Whether a list serves a ray's steps well is known only on the
+// way: steps long against a cell, of a loose tolerance away from the cores, use a
+// list once and are walked; short ones, and steps through dense cells, which one
+// thread would scan while the others wait, are left to the lists. A launch of many
+// rays therefore walks first and marks the rays it leaves; the list kernel takes
+// these from their start, in its own order (the costliest first; a few steps each
+// are done twice). Projections of 262,144 cells, lists alone -> walk and lists, in ms
+// (the walk alone, as it was before there were lists): outer 500 kpc at rtol 1e-2
+// 256^2 5.6 -> 3.1 (3.2), 512^2 20.7 -> 5.9 (6.4), 1024^2 79.6 -> 16.9 (18.7), at 2e-3
+// 10 -> 10 (17), 36 -> 13 (20), 137 -> 39 (41), at 1e-3 42 -> 42 (92), 129 -> 127 (154);
+// 2 Mpc through the core at 1e-2: 43 -> 45 (531), 113 -> 70 (507), 422 -> 183 (418).
+// Band map of 4,194,304 cells, 500 kpc, 1e-2, 1024^2: 111 -> 38 (45). 32 channels of
+// the outer slab, 512^2, 1e-2: 80 -> 29 (31); adjoint of a 256^2 map, 100 kpc, 1e-2:
+// 11.5 -> 6.4 (6.1). The walk's kernels take 4 blocks of 128 threads per SM (128
+// registers).
+// ---------------------------------------------------------------------------
+// What the list kernels take from their queue: all rays, or those left.
+__device__ __forceinline__ unsigned long long list_rays(const LeaveRule& r,
+                                                        unsigned long long all) {
+  return r.left ? *r.n_left : all;
+}
+__device__ __forceinline__ unsigned long long list_ray(const LeaveRule& r, unsigned long long q) {
+  return r.left ? r.list[q] : q;
+}
+
+// A ray begins with short steps whatever its tolerance (h = 1, then the least one,
+// 0.2), which grow by the step. Looks at the pace come every kNextLook steps, the
+// first three by rules of their own.
+constexpr uint32_t kNextLook = 8, kFirstLook = 8, kSecondLook = 16, kThirdLook = 24;
+constexpr uint32_t kDenseStep = 512;  // scans of a step's 4 points
+
+struct Pace {
+  float z;
+  uint32_t next;
+};
+
+__device__ __forceinline__ Pace pace_start(float z) { return Pace{z, kFirstLook}; }
+
+// After a step of a ray to z_end that ended at z, with the next one h, and made
+// `scans` scans: is the ray to be left?
+__device__ __forceinline__ bool pace_slow(Pace& p, const LeaveRule& r, float z, float z_end,
+                                          float h, unsigned long long steps, uint32_t scans) {
+  if (z + h >= z_end) return false;  // the last step
+  if (scans > kDenseStep) return true;
+  if (steps < p.next) return false;
+  float rays = r.rays, pace = (z - p.z) / (float)kNextLook;
+  // What the steps grow to: h after 8 and 16 steps is 0.21 and 0.28 at rtol 1e-3, 0.34
+  // and 0.9 at 1.5e-3, 0.5 and 2 at 2e-3, 1 and 7 at 3e-3, 6 and 100 (the largest step)
+  // at 1e-2, and the later mean steps are some 1, 7, 11, 15 and 25.
+  if (p.next == kFirstLook) {
+    pace = (h * h) * (h * h) / (kHmin * kHmin * kHmin);
+  } else if (p.next == kSecondLook) {
+    pace = 2.0f * h;
+  } else if (p.next != kThirdLook) {
+    // The rays still under way are those the lists would get. They make their steps
+    // again: the more there are of these against those still to come, the dearer.
+    rays -= (float)*(volatile unsigned long long*)r.done;
+    rays *= 1.0f + (float)steps * pace / (z_end - z);
+  }
+  p.z = z;
+  p.next += kNextLook;
+  return pace < fmaxf(r.even / fmaxf(rays - r.line, 1.0f), r.least);
+}
+
+// The ray of a 16 x 8 tile that this thread walks, in the list kernels' numbering (4 x
+// 2 pixels in a row of 8 rays): each warp an 8 x 4 block of pixels, so its 32 rays are
+// neighbours.
+__device__ __forceinline__ unsigned walk_ray() {
+  const unsigned warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, b = lane >> 3;
+  const unsigned sub = (2 * (warp >> 1) + (b >> 1)) * 4 + 2 * (warp & 1u) + (b & 1u);
+  return 8 * sub + (lane & 7u);
+}
+
+// The marks of a warp's rays, 8 of which in a row have numbers in a row.
+__device__ __forceinline__ void mark_left(const LeaveRule& r, bool active, bool leave,
+                                          unsigned long long ray, int lane) {
+  const unsigned m = __ballot_sync(kAll, leave), n = __popc(__ballot_sync(kAll, active));
+  if ((lane & 7) == 0) r.left[ray >> 3] = (uint8_t)(m >> lane);
+  if (lane == 0) atomicAdd(r.done, (unsigned long long)n);
 }
 
 }  // namespace ilc
