@@ -740,6 +740,22 @@ cudaError_t enqueue(Context& c, const BatchK& k, const GridView& g, int blocks, 
 
 }  // namespace
 
+cudaError_t batched_residency(int n_channels, int occ, int* id) {
+  Context c;  // (only its device is read)
+  cudaError_t e;
+  BatchK k{};
+  k.V = n_channels;
+  GridView g{};
+  int lists = 0, walk = 0;
+  if ((e = cudaGetDevice(&c.device)) ||
+      (e = n_channels > 1 ? persistent_blocks<true>(c, occ, &lists)
+                          : persistent_blocks<false>(c, occ, &lists)) ||
+      (e = walk_blocks(c, walk_kernel(k, g), occ, &walk)))
+    return e;
+  *id = 4096 * lists + walk;
+  return cudaSuccess;
+}
+
 cudaError_t channels_sort_launch(Context& c, const float* in, uint64_t n, int V, float* out) {
   const uint64_t total = n * (uint64_t)V;
   const unsigned blocks = (unsigned)std::min<uint64_t>((total + 255) / 256, 148ull * 16);

@@ -1291,31 +1291,37 @@ ilc_status ilc_autotune_render(ilc_ctx* h, const ilc_camera* cam, double z_range
   a.row_stride = sample_stride;
   ILC_CUDA(c, c.out_b.ensure((size_t)a.nx * (size_t)a.ny * 4), "autotune image");
   a.out = c.out_b.as<float>();
-  float best_ms = 0.0f;
-  bool first = true;
   for (int32_t i = 0; i < n_windows; ++i) {
     if (!(windows[i] >= 0.0f) || !std::isfinite(windows[i]))
       return fail(c, ILC_ERR_INVALID_ARGUMENT, "invalid z window candidate");
-    for (int32_t j = 0; j < n_occupancies; ++j) {
+    for (int32_t j = 0; j < n_occupancies; ++j)
       if (occupancies[j] != 0 && occupancies[j] != 3 && occupancies[j] != 4 && occupancies[j] != 5)
         return fail(c, ILC_ERR_INVALID_ARGUMENT, "occupancy must be 0, 3, 4 or 5");
+  }
+  // the window has no effect: one launch for each way the kernels can be resident,
+  // its time for all pairs that come to it, the first of the fastest ones wins
+  std::vector<int> ids((size_t)n_occupancies);
+  std::vector<float> ms((size_t)n_occupancies, 0.0f);
+  int32_t best = 0;
+  for (int32_t j = 0; j < n_occupancies; ++j) {
+    ILC_CUDA(c, render_residency(occupancies[j], &ids[j]), "autotune residency");
+    const int32_t same = (int32_t)(std::find(ids.begin(), ids.begin() + j, ids[j]) - ids.begin());
+    if (same < j) {
+      ms[j] = ms[same];
+    } else {
       a.occupancy_override = occupancies[j];
-      float ms = 0.0f;
-      ILC_CUDA(c, render_launch(c, a, &ms), "autotune render");
+      ILC_CUDA(c, render_launch(c, a, &ms[j]), "autotune render");
       uint32_t flags = 0;
       ilc_status st = read_flags(c, &flags, nullptr);
       if (st) return st;
       if (flags & FLAG_STEP_LIMIT)
         return fail(c, ILC_ERR_STEP_LIMIT, "rays reached the per-ray step limit");
-      if (times_ms) times_ms[i * n_occupancies + j] = ms;
-      if (first || ms < best_ms) {
-        first = false;
-        best_ms = ms;
-        *best_window = windows[i];
-        *best_occupancy = occupancies[j];
-      }
+      if (ms[j] < ms[best]) best = j;
     }
+    for (int32_t i = 0; times_ms && i < n_windows; ++i) times_ms[i * n_occupancies + j] = ms[j];
   }
+  *best_window = windows[0];
+  *best_occupancy = occupancies[best];
   c.render_occupancy = *best_occupancy;
   return ILC_OK;
 }
@@ -1438,11 +1444,20 @@ ilc_status ilc_autotune_batched(ilc_ctx* h, const float* values, int32_t n_chann
     c.batch_occupancy = keep_o;
     c.batch_cost_order = keep_order;
   };
+  // (as in ilc_autotune_render, for every tile width)
+  std::vector<int> ids((size_t)n_occupancies);
+  for (int32_t j = 0; j < n_occupancies; ++j)
+    ILC_CUDA(c, batched_residency(n_channels, occupancies[j], &ids[j]), "autotune residency");
+  std::vector<float> ms((size_t)n_occupancies);
   float best = 0.0f;
   bool first = true;
   for (int32_t i = 0; i < n_tiles; ++i) {
     for (int32_t j = 0; j < n_occupancies; ++j) {
-      for (int32_t q = 0; q < n_windows; ++q) {
+      const int32_t same =
+          (int32_t)(std::find(ids.begin(), ids.begin() + j, ids[j]) - ids.begin());
+      if (same < j) {
+        ms[j] = ms[same];
+      } else {
         c.batch_tile_w = tile_ws[i];
         c.batch_occupancy = occupancies[j];
         c.batch_cost_order = true;
@@ -1455,8 +1470,7 @@ ilc_status ilc_autotune_batched(ilc_ctx* h, const float* values, int32_t n_chann
         }
         ILC_CUDA(c, c.out_b.ensure(len * 4), "autotune images");
         a.out = c.out_b.as<float>();
-        float ms = 0.0f;
-        ILC_CUDA(c, batched_launch(c, a, &ms), "autotune batched kernel");
+        ILC_CUDA(c, batched_launch(c, a, &ms[j]), "autotune batched kernel");
         uint32_t flags = 0;
         st = read_flags(c, &flags, nullptr);
         if (st) {
@@ -1467,17 +1481,18 @@ ilc_status ilc_autotune_batched(ilc_ctx* h, const float* values, int32_t n_chann
           restore();
           return fail(c, ILC_ERR_STEP_LIMIT, "rays reached the per-ray step limit");
         }
-        if (times_ms) times_ms[(i * n_occupancies + j) * n_windows + q] = ms;
-        if (first || ms < best) {
+        if (first || ms[j] < best) {
           first = false;
-          best = ms;
+          best = ms[j];
           *best_tile_w = tile_ws[i];
           *best_occupancy = occupancies[j];
-          *best_window = windows[q];
         }
       }
+      for (int32_t q = 0; times_ms && q < n_windows; ++q)
+        times_ms[(i * n_occupancies + j) * n_windows + q] = ms[j];
     }
   }
+  *best_window = windows[0];
   c.batch_tile_w = *best_tile_w;
   c.batch_occupancy = *best_occupancy;
   c.batch_cost_order = true;

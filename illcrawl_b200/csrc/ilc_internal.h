@@ -262,6 +262,10 @@ cudaError_t adjoint_ray_launch(Context& c, const RenderArgs& a, int mode, const 
 cudaError_t adjoint_chain_launch(Context& c, const double* grad, uint64_t n, const float* dq_lnrho,
                                  const float* dq_lnT, float* g_lnrho, float* g_lnT);
 cudaError_t render_launch(Context& c, const RenderArgs& a, float* kernel_ms);
+// Blocks per SM of a render's (a batched render's) kernels under the occupancy `occ`,
+// one number for all of them: equal numbers, equal launches.
+cudaError_t render_residency(int occ, int* id);
+cudaError_t batched_residency(int n_channels, int occ, int* id);
 LeaveRule walk_rule(Context& c, double rays, unsigned long long n_rays,
                     unsigned long long* queue);
 // The list of the rays marked, in their order.

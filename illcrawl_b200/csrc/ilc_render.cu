@@ -458,6 +458,20 @@ cudaError_t left_list_launch(Context& c, const LeaveRule& r) {
   return cudaGetLastError();
 }
 
+cudaError_t render_residency(int occ, int* id) {
+  cudaError_t e;
+  int lists = 0, walk = 0;
+  if ((e = cudaFuncSetAttribute(render_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)sizeof(RenderMem))) ||
+      (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&lists, render_kernel, kListThreads,
+                                                         sizeof(RenderMem))) ||
+      (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&walk, walk_kernel<false>,
+                                                         kSlotThreads, 0)))
+    return e;
+  *id = occ > 0 ? 64 * std::min(lists, occ) + std::min(walk, occ) : 64 * lists + walk;
+  return cudaSuccess;
+}
+
 cudaError_t render_launch(Context& c, const RenderArgs& a, float* kernel_ms) {
   cudaError_t e;
   if ((e = c.flags.ensure(kFlagsBytes))) return e;

@@ -502,15 +502,15 @@ ilc_status ilc_render_batched(ilc_ctx* ctx, const float* values, int32_t n_chann
  * cost_order != 0 hands out the tiles in decreasing order of an
  * estimated cost (particles projected into each tile's columns, weighted by
  * their cell's occupancy), so the longest rays start first. Changes the order
- * of work only, never a result. Default: 8, 4, 40, 1. */
+ * of work only, never a result. Default: 8, 4, any z_window, 1. */
 ilc_status ilc_set_batch_schedule(ilc_ctx* ctx, int32_t tile_w, int32_t blocks_per_sm,
                                   float z_window, int32_t cost_order);
 
 /* Autotuner of the batched render's schedule: renders the jobs once per
  * (tile_w, occupancy, z_window) candidate (outputs discarded, cost order on),
- * times the kernel with CUDA events, sets the fastest and returns it
+ * times the kernels with CUDA events, sets the fastest and returns it
  * (times_ms, may be NULL: n_tiles x n_occupancies x n_windows, in that
- * nesting). Callers pass a representative subset of their jobs (e.g. the
+ * nesting; equal launches once, as in ilc_autotune_render). Callers pass a representative subset of their jobs (e.g. the
  * same cameras at a lower resolution). */
 ilc_status ilc_autotune_batched(ilc_ctx* ctx, const float* values, int32_t n_channels,
                                 int values_on_device, const ilc_job* jobs, int32_t n_jobs,
@@ -560,11 +560,13 @@ ilc_status ilc_adjoint_xray_flux(ilc_ctx* ctx, const float* cells, const float* 
                                  ilc_adjoint_stats* stats);
 
 /* Autotuner of the adaptive render's schedule: renders every sample_stride-th
- * row of 8-pixel tiles of the view once per (z window, occupancy) candidate
- * pair, times the render kernel with CUDA events, sets the fastest pair on the
+ * row of 8-pixel tiles of the view for each (z window, occupancy) candidate
+ * pair, times the render's kernels with CUDA events, sets the fastest pair on the
  * context and returns it (times_ms, may be NULL: n_windows x n_occupancies
- * kernel times, window-major). Needs the particles set up. The result depends
- * on the particle distribution and the view, so callers cache it per workload. */
+ * kernel times, window-major). Pairs that come to the same launch (windows, and
+ * occupancies above what is resident) are timed once and share the time; the first
+ * of them is returned. Needs the particles set up. The result depends on the
+ * particle distribution and the view, so callers cache it per workload. */
 ilc_status ilc_autotune_render(ilc_ctx* ctx, const ilc_camera* cam, double z_range,
                                ilc_tolerance tol, int32_t controller, const float* windows,
                                int32_t n_windows, const int32_t* occupancies,
