@@ -116,8 +116,11 @@ __device__ __forceinline__ EmitCall emit_call(const GauntView& G, float r) {
   k.r = r;
   k.r2 = r * r;
   k.yr2 = 1.0f / k.r2;
-  k.ok = G.pad == kPad && G.dy >= 1e-6f && G.dy <= 1e6f && fabsf(G.y0) <= 1e6f && k.r2 >= 1e-12f &&
-         k.r2 <= 1e15f;
+  // (r from 1e-10 to 1e10 in any unit: a luminosity distance is 3e7 kpc at redshift
+  // 3.5 and 1e8 at 10; with brems for every cell, 1,000,000 cells take 210 us instead
+  // of 91)
+  k.ok = G.pad == kPad && G.dy >= 1e-6f && G.dy <= 1e6f && fabsf(G.y0) <= 1e6f && k.r2 >= 1e-20f &&
+         k.r2 <= 1e20f;
   k.vmin = fmaxf(1e-20f, 1e-26f * k.r2);
   k.vmax = fminf(1e28f, 1e26f * k.r2);
   return k;

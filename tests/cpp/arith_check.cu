@@ -126,7 +126,7 @@ int main() {
   rc |= report("div_by");
   div_kernel<<<blocks, 256>>>(many, 2ull << 40, -24, 20, -20, 19, 0.0f, 3e38f, counts, counts + 1);
   rc |= report("div_by");
-  div_kernel<<<blocks, 256>>>(many, 3ull << 40, -66, 93, -39, 49, 1e-26f, 1e26f, counts,
+  div_kernel<<<blocks, 256>>>(many, 3ull << 40, -66, 93, -66, 66, 1e-26f, 1e26f, counts,
                               counts + 1);
   rc |= report("div_by");
   div_kernel<<<blocks, 256>>>(many, 4ull << 40, -86, 86, -26, 26, 1e-34f, 1e34f, counts,
