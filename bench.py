@@ -144,8 +144,8 @@ def tune_schedule(ctx, cam, args, gpu_name):
         half = ilc.camera(*camera_args()[:4], NX // 2, NY // 2)
         q = ctx.tuning_values
         bt, bo, bw, times = ctx.autotune_batched(q, [ilc.job(half, z_range=DEPTH)], REL_TOL, 0.0,
-                                                 tile_ws=(0, 4, 8), occupancies=(4, 5),
-                                                 windows=(20.0, 80.0))
+                                                 tile_ws=(0, 4, 8), occupancies=(3, 4),
+                                                 windows=(0.0,))
         cache[key] = {"tile_w": bt, "occupancy": bo, "z_window": bw,
                       "kernel_ms": {f"t{t}_o{o}_w{w}": v for (t, o, w), v in times.items()}}
         src = "autotuner"
@@ -324,7 +324,7 @@ def spectral_schedule(ctx, ilc, tab, gpu_name, args):
     small = spectrum_jobs(ilc, 4)
     tune_jobs = [small[i] for i in SPECTRAL_SUBSET]
     bt, bo, bw, times = ctx.autotune_batched(tab, tune_jobs, REL_TOL, 0.0, tile_ws=(0, 4, 8),
-                                             occupancies=(0, 4), windows=(40.0, 160.0))
+                                             occupancies=(3, 4), windows=(0.0,))
     cache[key] = {"tile_w": bt, "occupancy": bo, "z_window": bw,
                   "kernel_ms": {f"t{t}_o{o}_w{w}": v for (t, o, w), v in times.items()}}
     try:

@@ -297,7 +297,7 @@ adjoint_kernel(const __grid_constant__ AdjK a, const __grid_constant__ GridView 
     eval_points<true>(g, M.spiral, W, lane, go && !(replay && pj == 3), px, py, pz, lx,
                                ly, lz, zq, h, s, ws);
     ScatterSlots cur;
-    if (go) scatter_slots(s, cur);
+    if (go && !(replay && pj == 3)) scatter_slots(s, cur);
     bool accepted = go;
     const float hb = h;
     if (replay) {

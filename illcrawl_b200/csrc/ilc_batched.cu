@@ -671,8 +671,10 @@ __global__ void tile_cost_kernel(const float4* __restrict__ parts,
   }
 }
 
-// One channel: 4 blocks of 128 threads per SM (126 registers, 54 KB of shared
-// memory); V > 1 adds the hand-over and runs 3.
+// One channel: 4 blocks of 128 threads per SM, by registers (128) and shared memory
+// (227 KB); V > 1 adds the hand-over and runs 3.
+static_assert(sizeof(BlockMem<false>) <= 50 * 1024 && sizeof(BlockMem<true>) <= 57 * 1024,
+              "4 and 3 blocks per SM, with shared memory left for L1");
 template <bool kMulti> struct Variant {
   static constexpr int kBlocks = kMulti ? 3 : 4;
   static constexpr size_t kSmem = sizeof(BlockMem<kMulti>);

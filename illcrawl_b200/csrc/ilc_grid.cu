@@ -59,7 +59,7 @@ __global__ void bbox_kernel(const float4* __restrict__ in, uint64_t n, unsigned*
   }
   bad = __any_sync(0xffffffffu, bad);
   // one set of atomics per block: those of every warp queued up on the seven
-  // words (42 us of 1,000,003 particles' box; now 6)
+  // words (42 us of 1,000,003 particles' box; now 8)
   __shared__ unsigned part[32][7];
   if ((threadIdx.x & 31) == 0) {
 #pragma unroll
@@ -399,9 +399,9 @@ int radix_pass(const uint32_t* ka, const uint32_t* va, uint64_t n, int shift, ui
   return 2 + scans;
 }
 
-// Bits of a digit: 8, or up to 10 where that saves a pass (keys of 17 to 20
-// bits: grids of 131,073 to 1,048,576 cells) and the histogram stays small.
-// Sorting 1,000,003 keys of 17 bits takes 2 passes of 36 us instead of 3.
+// Bits of a digit: 8, or 9 or 10 where that saves a pass (keys of 9, 10, 17 to 20 and
+// 25 to 30 bits) and the histogram stays small. Sorting 1,000,003 keys of 17 bits
+// (131,073 cells or more) takes 2 passes of 36 us instead of 3.
 int digit_bits(int bits, uint64_t n) {
   const int p8 = (bits + 7) / 8, p10 = (bits + 9) / 10;
   if (p10 == p8 || n > (1ull << 23)) return 8;

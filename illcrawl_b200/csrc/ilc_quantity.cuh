@@ -12,7 +12,6 @@
 
 namespace ilc {
 
-constexpr int kMaxTable = 81 * 146;
 // The table with two rows and columns of zeros around it: a lookup next to or
 // outside the table then reads its zeros like any other texel. Very long or
 // wide tables, which would not fit shared memory that way, stay unpadded.
