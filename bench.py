@@ -101,10 +101,10 @@ TUNING_FILE = os.path.join(ROOT, "illcrawl_b200", "data", "render_tuning.json")
 
 def tune_schedule(ctx, cam, args, gpu_name):
     """Schedule of the render kernel (orders work only, never changes a
-    result). Persistent engine: tile shape, blocks per SM and z window from
-    the cache for this GPU and workload, else defaults; --autotune re-runs the
-    autotuner on the same camera at half resolution (8,192 tiles) and caches
-    the winner. Grid engine: z window and occupancy, likewise."""
+    result). Persistent engine: tile shape and blocks per SM (the z window has
+    no effect) from the cache for this GPU and workload, else defaults;
+    --autotune re-runs the autotuner on the same camera at half resolution
+    (8,192 tiles) and caches the winner. Grid engine: occupancy, likewise."""
     import illcrawl_b200 as ilc
     cache = json.load(open(TUNING_FILE)) if os.path.exists(TUNING_FILE) else {}
     base = f"{gpu_name}|xray_band_map_4M_cells_{NX}sq_rtol1e-3|z0={Z_START}|depth={DEPTH}"
@@ -723,9 +723,10 @@ def run_ours(args, rank, world, local_rank):
                      "kernel_ms": last_stats["kernel_ms"], "algorithmic_bytes": kbytes,
                      "bytes_source": bytes_provenance(last_stats),
                      "note": "algorithmic bytes of the survey's byte model (every candidate of "
-                             "every visited cell, per query); the kernel reads far fewer DRAM "
-                             "bytes (traffic) because the grid stays in L2 and one load serves "
-                             "4 points: the walk is latency-bound, not DRAM-bound"},
+                             "every visited cell, per query); the kernels read far fewer DRAM "
+                             "bytes (traffic) because the grid stays in L2 and a candidate list "
+                             "serves several steps: they are bound by instruction issue, not "
+                             "by DRAM"},
         "cpu_baseline": {"value": cpu_v, "unit": "Mrays/s", "cores": cores, "kind": "port",
                          "sample": "the oracle renders 2048 random rays of the 1024^2 map "
                                    "(adaptive, FP64 controller) after building the per-cell "
