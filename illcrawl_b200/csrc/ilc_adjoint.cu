@@ -390,7 +390,7 @@ adjoint_walk_kernel(const __grid_constant__ AdjK a, const __grid_constant__ Grid
     ScatterSlots prev;  // point 2 of the last accepted step: the next one's k1
     double prev_c = 0.0;
     bool have_prev = false;
-    WalkStats ws;
+    Walk4Stats ws;
     while ((int64_t)steps < limit && (replay || z < a.z_end)) {
       if (replay) h = hs[steps];
       float pts[4];

@@ -51,24 +51,26 @@ struct BatchK {
   float* walk_state;  // state of the walk kernel's rays, 4 V floats per thread
 };
 
-// Ray ti of work item `item`: its job and pixel; false outside the image.
-__device__ __forceinline__ bool item_pixel(const BatchK& a, const JobDev& J, uint64_t item, int ti,
+__device__ __forceinline__ int tile_rows(int tw) { return tw > 0 ? 32 / tw : 1; }
+
+// Ray ti of the job's work item t: its pixel; false outside the image. Compact tiles
+// are tw x th pixels, th = 32 / tw.
+__device__ __forceinline__ bool item_pixel(const JobDev& J, int tw, int th, uint64_t t, int ti,
                                            int& ix, int& iy) {
-  const uint64_t t = item - J.item_begin;
-  if (a.tile_w > 0) {  // compact tile of tile_w x (32 / tile_w) pixels
+  bool inside;
+  if (tw > 0) {
     const int tx = (int)(t % (uint64_t)J.tiles_x), ty = (int)(t / (uint64_t)J.tiles_x);
-    ix = tx * a.tile_w + ti % a.tile_w;
-    iy = ty * (32 / a.tile_w) + ti / a.tile_w;
-    return ix < J.nx && iy < J.ny;
+    ix = tx * tw + ti % tw;
+    iy = ty * th + ti / tw;
+    inside = ix < J.nx && iy < J.ny;
+  } else {  // strided: pixels t, t + T, t + 2T, ... (T = items of the job)
+    const uint64_t pix = t + (uint64_t)ti * (uint64_t)J.tiles_x;
+    inside = pix < (uint64_t)J.nx * (uint64_t)J.ny;
+    ix = inside ? (int)(pix % (uint64_t)J.nx) : J.nx;
+    iy = inside ? (int)(pix / (uint64_t)J.nx) : J.ny;
   }
-  // strided: pixels t, t + T, t + 2T, ... (T = items of the job)
-  const uint64_t pix = t + (uint64_t)ti * (uint64_t)J.tiles_x;
-  const bool inside = pix < (uint64_t)J.nx * (uint64_t)J.ny;
-  ix = inside ? (int)(pix % (uint64_t)J.nx) : J.nx;
-  iy = inside ? (int)(pix / (uint64_t)J.nx) : J.ny;
   return inside;
 }
-
 // Largest k with jobs[k].item_begin <= item.
 __device__ __forceinline__ int find_job(const JobDev* __restrict__ jobs, int n, uint64_t item) {
   int lo = 0, hi = n - 1;
@@ -156,21 +158,15 @@ struct ChanHand {
   float ws[4][kRays];   // sum of point j's weights
 };
 
-struct ListHand {
-  const ChanHand& h;
-  int r;
-  __device__ __forceinline__ float w(int p, int q) const { return h.w[p * 8 + q][r]; }
-  __device__ __forceinline__ int id(int p, int q) const { return h.id[p * 8 + q][r]; }
-  __device__ __forceinline__ float ws(int p) const { return h.ws[p][r]; }
-};
-
 // The step (zr, hr) of one ray for all channels, by a whole warp: the channels'
-// values at the 4 points (from the slots' weights and indices in H), the joint step
-// control, and the ray's state (I[V], k1[V] and room for their candidates) if the
-// step is accepted. nh: the next step size.
-template <class Hand>
-__device__ __forceinline__ bool channels_step(const BatchK& a, const Hand& H, float* Is, float zr,
-                                              float hr, int lane, double& nh) {
+// values at the 4 points, the joint step control, and the ray's state (I[V], k1[V] and
+// room for their candidates) if the step is accepted. w, ids, sums: the ray's column
+// of slot weights, indices (32 rows 8 j + t) and sums of weights (4 rows), kStride
+// words apart. nh: the next step size.
+template <int kStride>
+__device__ __forceinline__ bool channels_step(const BatchK& a, const float* w, const int* ids,
+                                              const float* sums, float* Is, float zr, float hr,
+                                              int lane, double& nh) {
   float* Ks = Is + a.V;
   const double hd = (double)hr;
   const double zd = (double)(zr + hr), rz = 1.0 / zd;
@@ -203,16 +199,16 @@ __device__ __forceinline__ bool channels_step(const BatchK& a, const Hand& H, fl
         float dot[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
-          const int id = H.id(p, q);
+          const int id = ids[(p * 8 + q) * kStride];
           const float4 v = id >= 0 ? __ldg(&chan4[(size_t)id * G + gi])
                                    : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-          const float wq = H.w(p, q);
+          const float wq = w[(p * 8 + q) * kStride];
           dot[0] = __fmaf_rn(wq, v.x, dot[0]);
           dot[1] = __fmaf_rn(wq, v.y, dot[1]);
           dot[2] = __fmaf_rn(wq, v.z, dot[2]);
           dot[3] = __fmaf_rn(wq, v.w, dot[3]);
         }
-        const float wsum = H.ws(p);
+        const float wsum = sums[p * kStride];
 #pragma unroll
         for (int k = 0; k < 4; ++k)
           ev[p][k] = (wsum != 0.0f && dot[k] != 0.0f) ? dot[k] / wsum : 0.0f;
@@ -239,11 +235,11 @@ __device__ __forceinline__ bool channels_step(const BatchK& a, const Hand& H, fl
         float dot = 0.0f;
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
-          const int id = H.id(p, q);
+          const int id = ids[(p * 8 + q) * kStride];
           const float v = id >= 0 ? __ldg(&a.chan[(size_t)id * a.V + c]) : 0.0f;
-          dot = __fmaf_rn(H.w(p, q), v, dot);
+          dot = __fmaf_rn(w[(p * 8 + q) * kStride], v, dot);
         }
-        const float wsum = H.ws(p);
+        const float wsum = sums[p * kStride];
         ev[p] = (wsum != 0.0f && dot != 0.0f) ? dot / wsum : 0.0f;
       }
       double x;
@@ -318,6 +314,9 @@ batched_kernel(const __grid_constant__ BatchK a, const __grid_constant__ GridVie
   const unsigned wg = blockIdx.x * kListWarps + warp;
   if (lane == 0) W.over = a.over + (size_t)wg * kRays * kOver;
   ChanHand& H = M.hand[kMulti ? warp : 0];
+  // (kept with V > 1: spectra of 16^2 pixels lose 4 % to the division at each ray; with
+  // V = 1 the register is worth more)
+  const int tw = a.tile_w, th = tile_rows(tw);
   float* wstate = kMulti ? a.state + ((size_t)blockIdx.x * kListThreads / 4 +
                                       (size_t)warp * kRays) * 4 * (size_t)a.V
                          : nullptr;
@@ -345,7 +344,8 @@ batched_kernel(const __grid_constant__ BatchK a, const __grid_constant__ GridVie
           const uint64_t item = a.order ? (uint64_t)a.order[qi] : qi;
           const JobDev& J = a.jobs[find_job(a.jobs, a.n_jobs, item)];
           int ix, iy;
-          const bool inside = item_pixel(a, J, item, (int)(ray & 31), ix, iy);
+          const bool inside = item_pixel(J, tw, kMulti ? th : tile_rows(tw),
+                                         item - J.item_begin, (int)(ray & 31), ix, iy);
           if (inside) {
             bool masked;
             float o[3];
@@ -420,8 +420,9 @@ batched_kernel(const __grid_constant__ BatchK a, const __grid_constant__ GridVie
         gom &= gom - 1;
         const float zr = __shfl_sync(kAll, z, gl), hr = __shfl_sync(kAll, h, gl);
         double nh;
-        const bool accept = channels_step(
-            a, ListHand{H, tr}, wstate + (size_t)tr * 4 * a.V, zr, hr, lane, nh);
+        const bool accept =
+            channels_step<kRays>(a, &H.w[0][tr], &H.id[0][tr], &H.ws[0][tr],
+                                 wstate + (size_t)tr * 4 * a.V, zr, hr, lane, nh);
         if (r == tr) {
           my_acc = accept;
           my_nh = nh;
@@ -472,19 +473,6 @@ batched_kernel(const __grid_constant__ BatchK a, const __grid_constant__ GridVie
   }
 }
 
-// V > 1, a walked ray: weights in the distance rows of its slot columns, indices in
-// the value rows.
-struct WalkHand {
-  const SlotMem& m;
-  const float (*sum)[kSlotThreads];
-  int t;
-  __device__ __forceinline__ float w(int p, int q) const { return m.d[p * 8 + q][t]; }
-  __device__ __forceinline__ int id(int p, int q) const {
-    return __float_as_int(m.v[p * 8 + q][t]);
-  }
-  __device__ __forceinline__ float ws(int p) const { return sum[p][t]; }
-};
-
 // Point J's slots to weights in place (the indices stay), and their sum.
 template <int J> __device__ __forceinline__ void slots_to_weights(const Step4& s, float& sum) {
   float w[8], ws;
@@ -510,6 +498,7 @@ batched_walk_kernel(const __grid_constant__ BatchK a, const __grid_constant__ Gr
   if (threadIdx.x < 7) blk[threadIdx.x] = 0ull;
   load_spiral(spiral, spiral_g);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int tw = a.tile_w, th = tile_rows(tw);
   float* wstate = kMulti ? a.walk_state + ((size_t)blockIdx.x * kSlotThreads +
                                            (size_t)warp * 32) * 4 * (size_t)a.V
                          : nullptr;
@@ -521,7 +510,7 @@ batched_walk_kernel(const __grid_constant__ BatchK a, const __grid_constant__ Gr
     const uint64_t item = a.order ? (uint64_t)a.order[turn] : turn;
     const JobDev& J = a.jobs[find_job(a.jobs, a.n_jobs, item)];
     int ix, iy;
-    const bool inside = item_pixel(a, J, item, lane, ix, iy);
+    const bool inside = item_pixel(J, tw, th, item - J.item_begin, lane, ix, iy);
     bool masked = true;
     float o[3] = {0.0f, 0.0f, 0.0f}, len = 0.0f;
     if (inside) ray_span(J, ix, iy, masked, o, len);
@@ -529,7 +518,7 @@ batched_walk_kernel(const __grid_constant__ BatchK a, const __grid_constant__ Gr
     bool run = inside && !masked, leave = false;
     float z = 0.0f, h = 1.0f, I = 0.0f, k1 = 0.0f;
     uint32_t rs = 0, ra = 0;
-    WalkStats ws;
+    Walk4Stats ws;
     Pace pace = pace_start(0.0f);
     if (kMulti) {
       for (int i = lane; i < 32 * 4 * a.V; i += 32) wstate[i] = 0.0f;
@@ -571,10 +560,13 @@ batched_walk_kernel(const __grid_constant__ BatchK a, const __grid_constant__ Gr
           const int r = __ffs(gom) - 1;
           gom &= gom - 1;
           const float zr = __shfl_sync(kAll, z, r), hr = __shfl_sync(kAll, h, r);
+          const int t = warp * 32 + r;  // ray r's slot columns: weights, indices
           double nh;
           const bool accept =
-              channels_step(a, WalkHand{slot_mem, slot_ws, warp * 32 + r},
-                            wstate + (size_t)r * 4 * a.V, zr, hr, lane, nh);
+              channels_step<kSlotThreads>(a, &slot_mem.d[0][t],
+                                          reinterpret_cast<const int*>(&slot_mem.v[0][t]),
+                                          &slot_ws[0][t], wstate + (size_t)r * 4 * a.V, zr, hr,
+                                          lane, nh);
           if (lane == r) {
             my_acc = accept;
             my_nh = nh;

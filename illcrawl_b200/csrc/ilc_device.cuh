@@ -97,7 +97,6 @@ struct GridView {
 struct WalkStats {
   uint32_t cells = 0;
   uint32_t cands = 0;
-  uint32_t scans = 0;  // of a step's walk: candidates scanned, a quarter of those behind codes
 };
 
 // Slot state of one query: the reference's 8-entry (distance, value) lists.

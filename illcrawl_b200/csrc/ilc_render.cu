@@ -252,7 +252,7 @@ __device__ __forceinline__ void walk_tile(const RenderK& a, const GridView& g,
   int ix, iy;
   ray_pixel(a, q, ix, iy);
   const bool active = ix < a.cam.nx && iy < a.row_end;
-  WalkStats ws;
+  Walk4Stats ws;
   unsigned long long steps = 0, acc = 0, at_limit = 0;
   bool leave = false;
   if (active) {
@@ -310,7 +310,7 @@ __device__ __forceinline__ void walk_tile(const RenderK& a, const GridView& g,
     }
     if (leave) {
       steps = acc = 0;
-      ws = WalkStats();
+      ws = Walk4Stats();
     } else {
       const size_t pix = (size_t)iy * a.cam.nx + ix;
       if (a.out) a.out[pix] = a.apply_scale ? I * a.scale : I;

@@ -38,6 +38,11 @@ struct SlotMem {
   float v[kSlotRows][kSlotThreads];
 };
 
+// Counters of a walked ray.
+struct Walk4Stats : WalkStats {
+  uint32_t scans = 0;  // candidates scanned, a quarter of those behind codes
+};
+
 struct Step4 {
   float qx[4], qy[4], qz[4];
   float* sd;      // this thread's distance column: sd[(j * 8 + t) * kSlotThreads]
@@ -244,7 +249,7 @@ __device__ __forceinline__ bool prune_range(const GridView& g, int ix, int iy, i
 template <bool kSharedXY, bool kIdx>
 __device__ __forceinline__ void walk4(const GridView& g, const char4* __restrict__ spiral,
                                       Step4& s, unsigned mask, int cx, int cy, int cz, int sub,
-                                      WalkStats& st) {
+                                      Walk4Stats& st) {
   const char4* order = spiral + sub * 125;
   unsigned act = mask;
   float thr[4];
@@ -356,7 +361,7 @@ template <bool kIdx>
 __device__ __forceinline__ void nn8_walk_step4(const GridView& g,
                                                const char4* __restrict__ spiral, float px,
                                                float py, float pz, float lx, float ly, float lz,
-                                               const float zq[4], Step4& s, WalkStats& st) {
+                                               const float zq[4], Step4& s, Walk4Stats& st) {
   int cx[4], cy[4], cz[4], sb[4];
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
@@ -415,7 +420,7 @@ template <bool kIdx>
 __device__ __forceinline__ void nn8_step4(const GridView& g, const char4* __restrict__ spiral,
                                           SlotMem& sm, float px, float py, float pz, float lx,
                                           float ly, float lz, const float zq[4], float e[4],
-                                          WalkStats& st) {
+                                          Walk4Stats& st) {
   Step4 s;
   s4_bind(s, sm);
   nn8_walk_step4<kIdx>(g, spiral, px, py, pz, lx, ly, lz, zq, s, st);
