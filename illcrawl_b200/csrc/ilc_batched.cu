@@ -587,7 +587,8 @@ batched_walk_kernel(const __grid_constant__ BatchK a, const __grid_constant__ Gr
         run = false;
       }
     }
-    mark_left(a.leave, inside && !masked, leave, 32 * turn + lane, lane);
+    const bool counted = inside && !masked && !(J.radius > 0.0);  // as in BatchArgs::rays
+    mark_left(a.leave, counted, leave, 32 * turn + lane, lane);
     if (!kMulti) {
       if (inside && !leave)
         a.out[J.out_offset + (size_t)iy * J.nx + ix] = masked ? 0.0f : I * J.scale;

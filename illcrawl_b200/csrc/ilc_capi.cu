@@ -263,8 +263,12 @@ ilc_status batched_jobs(Context& c, int32_t V, const ilc_job* jobs, int32_t n_jo
     d.scale = j.scale;
     d.out_offset = j.out_offset;
     d.item_begin = items;
+    // Rays that walk_rule() counts: inside the aperture, and not on chords, which lead
+    // through the core that their sphere surrounds, where lists are ahead (12 cameras of
+    // 128^2 x 130 bins at rtol 1e-2: 300 ms, and 342 ms walked first; 994 ms walked only).
     const double r = d.aperture / d.ps_d;  // the aperture's radius in pixels
-    rays += d.aperture > 0.0 ? std::min((double)npix, 3.14159265 * r * r) : (double)npix;
+    if (!chord)
+      rays += d.aperture > 0.0 ? std::min((double)npix, 3.14159265 * r * r) : (double)npix;
     items += tw > 0 ? (uint64_t)d.tiles_x * (uint64_t)((d.ny + th - 1) / th)
                     : (uint64_t)d.tiles_x;
   }

@@ -52,8 +52,8 @@ struct LeaveRule {
   // fewer rays than `line` lists are always ahead), and with the chip full of
   // short ones, `least`.
   float even, line, least;
-  float rays;                // of the launch, without masked ones
-  unsigned long long* done;  // of them, ended or left
+  float rays;                // of the launch, without masked ones and chords
+  unsigned long long* done;  // rays ended or left
   uint8_t* left;             // a bit per ray: left to the lists (nullptr: nothing is walked)
   uint64_t n_marks;
   uint32_t* list;            // the rays left, in their order
@@ -289,7 +289,7 @@ struct BatchArgs {
   const JobDev* jobs;     // device
   int32_t n_jobs;
   uint64_t n_items;
-  double rays;            // inside the apertures
+  double rays;            // inside the apertures of jobs without chords
   int32_t V;
   const float* chan;      // device, sorted order, n x V (V = 1: nullptr = particles' q)
   float* out;             // device images

@@ -102,6 +102,23 @@ def test_adaptive_walk_jobs(ctx, oracle_mod, rtol, tile_w):
         ctx.set_batch_schedule()
 
 
+def test_chords_take_lists(ctx, oracle_mod):
+    """Rays on chords through a core are not walked first, however many they are."""
+    import illcrawl_b200 as ilc
+    pts, g, args, depth = _setup(ctx, oracle_mod, "coded_cells")
+    vals = pts[:, 3].copy()
+
+    def jobs(m):
+        return [m.job(m.camera((50.0, 50.0, -10.0), Z, 0.1, 90.0, NX, NY), aperture_radius=44.0,
+                      sphere_center=(50.0, 50.0, 50.0), sphere_radius=40.0, min_chord=5.0)]
+
+    before = ctx.kernel_launches
+    img, st = ctx.render_batched(vals, jobs(ilc), rel_tol=2e-2)
+    assert ctx.kernel_launches - before == 3  # channel sort, cost, lists
+    want, ost, rc = oracle_mod.render_batched(g, vals, jobs(oracle_mod), 0.0, 2e-2)
+    assert rc == 0 and same_bits(img, want)
+
+
 def test_adaptive_walk_step_limit(ctx, oracle_mod):
     """Rays that reach the step limit are reported, walked or not."""
     import illcrawl_b200 as ilc
