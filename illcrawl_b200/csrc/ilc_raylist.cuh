@@ -49,7 +49,7 @@
 // arithmetic with 4 warps per scheduler (stalls of 2.3 cycles per issue) and
 // instruction fetch (2.0); the grid stays in L2 (DRAM 2 MB read per launch).
 // Images of very many rays gain less, since there the walks from scratch filled
-// the chip too: 1024^2 band map of 4,194,304 cells, 6 Mpc: 12.16 -> 10.77 s. Steps
+// the chip too: 1024^2 band map of 4,194,304 cells, 6 Mpc: 12.16 -> 10.55 s. Steps
 // that are long against a cell use a list once or twice, and lose: launches of many
 // rays walk those (ilc_walk4.cuh).
 #pragma once
