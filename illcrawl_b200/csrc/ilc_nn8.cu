@@ -616,15 +616,16 @@ cudaError_t query_order(Context& c, const GridView& g, const float4* pts, uint64
 constexpr uint64_t kThreadMin = 81920;
 // In an even grid (Context::even: particles in four of five cells or more, at most
 // a thousandth of them beyond the 48th of their cell) no lane's walk is long and
-// order gains little: from 40,960 queries on the lanes are ahead of the warps, and
+// order gains little: from 24,576 queries on the lanes are ahead of the warps, and
 // up to 393,216 the sort costs more than it saves. A few queries whose distances are
 // too close for squared ones would cost the warp kernel's latency (65,537 random
 // queries in 116 us, 81,000 in 135), so such grids are walked on rounded distances.
 // Whole calls in us, 100,000 uniform particles, random queries (in the order of their
-// cells): 65,537 by warps 165 (158), ordered lanes 135 (131), lanes 101 (86); 81,000:
+// cells): 16,384 by warps 68 (67), lanes 94 (80); 24,576: 84 (85), 88 (75); 36,000: 102
+// (99), 88 (78); 65,537: 165 (158), ordered lanes 135 (131), lanes 101 (86); 81,000:
 // 198 (192), 147 (142), 109 (92); 200,000: 439 (418), 189 (183), 168 (130); 394,000
 // ordered 235 (228), 393,000 unordered 246 (196).
-constexpr uint64_t kEvenMin = 40960, kEvenOrder = 393216;
+constexpr uint64_t kEvenMin = 24576, kEvenOrder = 393216;
 
 cudaError_t nn8_query_launch(Context& c, const float4* pts, uint64_t n, bool merge, float* out,
                              int32_t* idx8, float* d8) {

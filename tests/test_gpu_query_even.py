@@ -1,6 +1,6 @@
 """GPU parity of nn8 queries where nearly all grid cells hold particles and hardly
 any of them many, on both sides of the rule that takes them there (one warp per
-query below 40,960, one lane per query in the given order from there on, in the
+query below 24,576, one lane per query in the given order from there on, in the
 order of their bins from 393,216 on): slots, distances, values and search counters
 equal the oracle's, also with distances that tie, with a cell that is left to the
 warps, with queries on particles and outside the grid, and when a second block is
@@ -26,10 +26,10 @@ SETS = {"uniform": lambda: _uniform(30_000), "thousand": lambda: _uniform(1000),
         "duplicates": lambda: np.repeat(_uniform(10_000), 3, axis=0), "crowd": lambda: _crowd(120),
         "more_crowd": lambda: _crowd(200)}
 # one launch: warps; two: lanes, then warps for the rest; more: count, scan and order first
-LAUNCHES = {40_959: 1, 40_960: 2, 393_215: 2}
+LAUNCHES = {24_575: 1, 24_576: 2, 393_215: 2}
 
 
-@pytest.mark.parametrize("n", [40_959, 40_960, 393_215, 393_216])
+@pytest.mark.parametrize("n", [24_575, 24_576, 393_215, 393_216])
 @pytest.mark.parametrize("name", sorted(SETS))
 def test_query_even_bit_exact(ctx, oracle_mod, name, n):
     pts = SETS[name]()
@@ -55,7 +55,7 @@ def test_query_even_bit_exact(ctx, oracle_mod, name, n):
     assert stats == (int(ost[0]), int(ost[1]))
 
 
-@pytest.mark.parametrize("n", [40_960, 393_216])
+@pytest.mark.parametrize("n", [24_576, 393_216])
 def test_query_even_merge(ctx, oracle_mod, n):
     pts = np.random.default_rng(9).permutation(_crowd(200))
     a, b = pts[: len(pts) // 2], pts[len(pts) // 2:]
